@@ -517,8 +517,8 @@ class CudaOps:
         ids_e, off, slots = bufs["expert_ids"][:T], bufs["offsets"][:T], bufs["mapped_slots"][:T]
         scores = bufs["scores"][:T]
         k.moe_scatter(x, xs, ids_e, off, bufs["counts"], bufs["pad_off"], slots, f.top, scores if f.weighs_inputs else None)
-        k.moe_gemm(xs, lw.moe_up, bufs["pad_off"], E, hs, act=act, gated=f.gated, limit=f.limit)
-        k.moe_gemm(hs, lw.moe_down, bufs["pad_off"], E, ys)
+        k.moe_gemm(xs, lw.moe_up, bufs["pad_off"], E, hs, act=act, gated=f.gated, limit=f.limit, choices=T * f.top)
+        k.moe_gemm(hs, lw.moe_down, bufs["pad_off"], E, ys, choices=T * f.top)
         return k.moe_combine(ys, slots, None if f.weighs_inputs else scores, base, out)
 
     def table_moe(self, x, ids, lw, f, act, shared, out, bufs):

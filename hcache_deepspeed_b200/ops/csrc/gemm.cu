@@ -137,28 +137,28 @@ static bool skinny_enabled() {
     return on != 0;
 }
 
-template <int NT, int EPI, bool kBf16>
+template <int NT, int EPI, bool kBf16, bool kGrouped = false>
 static int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid,
                               cudaStream_t stream) {
-    auto kern = gemm_skinny_kernel<NT, EPI, kBf16>;
+    auto kern = gemm_skinny_kernel<NT, EPI, kBf16, false, kGrouped>;
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured[dev & 63]) {
         HDS_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            static_cast<int>(skinny_smem_bytes(NT))));
+                                            static_cast<int>(skinny_smem_bytes(NT, kGrouped))));
         configured[dev & 63] = true;
     }
-    HDS_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT), stream, tw, tx, a));
+    HDS_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT, kGrouped), stream, tw, tx, a));
     return HDS_OK;
 }
 
-template <int EPI, bool kBf16>
+template <int EPI, bool kBf16, bool kGrouped = false>
 static int launch_skinny_nt(int nt, const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid,
                             cudaStream_t stream) {
-    if (nt == 16) return launch_skinny_inst<16, EPI, kBf16>(tw, tx, a, grid, stream);
-    if (nt == 32) return launch_skinny_inst<32, EPI, kBf16>(tw, tx, a, grid, stream);
-    return launch_skinny_inst<64, EPI, kBf16>(tw, tx, a, grid, stream);
+    if (nt == 16) return launch_skinny_inst<16, EPI, kBf16, kGrouped>(tw, tx, a, grid, stream);
+    if (nt == 32) return launch_skinny_inst<32, EPI, kBf16, kGrouped>(tw, tx, a, grid, stream);
+    return launch_skinny_inst<64, EPI, kBf16, kGrouped>(tw, tx, a, grid, stream);
 }
 
 // One CTA per (128-feature tile, K split); splits fill the resident slots (SMs x CTAs per SM) once.
@@ -391,6 +391,44 @@ extern "C" int hds_gemm_accum(const void* A, int64_t lda, const void* W, int64_t
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     return dtype == 0 ? launch_gemm_bn<EPI_RED_F32, true>(bn, ops.ta, ops.tw, g, grid, s)
                       : launch_gemm_bn<EPI_RED_F32, false>(bn, ops.ta, ops.tw, g, grid, s);
+}
+
+/* The same for a decode step, where no expert has more than `max_per_expert` (<= 64) live rows: every weight is streamed once by
+   the feature-major kernel; rows past the live ones are written too, up to the token tile, inside the expert's own range. */
+extern "C" int hds_moe_gemm_few(const void* A, int64_t lda, const void* W_stacked, int64_t ldw, const int32_t* pad_off,
+                                int n_experts, int max_per_expert, int max_experts, int max_rows, int N, int K, int dtype, int epilogue,
+                                int act, void* out, int64_t ldo, void* stream) {
+    HDS_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_GATED, "hds_moe_gemm_few: epilogue must be 0 (store) or 1 (gated)");
+    HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_moe_gemm_few: dtype must be 0 (bf16) or 1 (fp16)");
+    HDS_REQUIRE(n_experts >= 1 && pad_off != nullptr && max_rows % kGemmBM == 0,
+                "hds_moe_gemm_few: needs expert offsets and a row capacity that is a multiple of 128");
+    HDS_REQUIRE(max_per_expert >= 1 && max_per_expert <= 64 && max_experts >= 1, "hds_moe_gemm_few: 1..64 rows per expert");
+    HDS_REQUIRE(N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0, "hds_moe_gemm_few: K, lda, ldw must be multiples of 8 elements");
+    HDS_REQUIRE(epilogue != EPI_GATED || (N % 2 == 0), "hds_moe_gemm_few: gated epilogue needs an even N");
+    const int nt = skinny_nt(max_per_expert);
+    const int n_tiles = (N + kSkinnyBF - 1) / kSkinnyBF;
+    SkinnyArgs a;
+    memset(&a, 0, sizeof(a));
+    a.M = max_per_expert; a.N = N; a.K = K;
+    a.splits = 1;
+    a.kb_per_split = (K + kGemmBK - 1) / kGemmBK;
+    a.act = act;
+    a.act_limit = gemm_take_act_limit();
+    a.out = out; a.ldo = ldo;
+    a.group_pad_off = pad_off;
+    a.n_groups = n_experts;
+    a.sync = tp_take_armed();
+    CUtensorMap tw, tx;
+    const bool bf16 = dtype == 0;
+    int rc = make_tmap_2d_16b(&tw, W_stacked, static_cast<uint64_t>(K), static_cast<uint64_t>(N) * n_experts,
+                              static_cast<uint64_t>(ldw) * 2, kGemmBK, kSkinnyBF, bf16);
+    if (rc) return rc;
+    rc = make_tmap_2d_16b(&tx, A, static_cast<uint64_t>(K), static_cast<uint64_t>(max_rows), static_cast<uint64_t>(lda) * 2, kGemmBK, nt, bf16);
+    if (rc) return rc;
+    const int grid = n_tiles * (max_experts < n_experts ? max_experts : n_experts);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (bf16) return epilogue == EPI_STORE ? launch_skinny_nt<EPI_STORE, true, true>(nt, tw, tx, a, grid, s) : launch_skinny_nt<EPI_GATED, true, true>(nt, tw, tx, a, grid, s);
+    return epilogue == EPI_STORE ? launch_skinny_nt<EPI_STORE, false, true>(nt, tw, tx, a, grid, s) : launch_skinny_nt<EPI_GATED, false, true>(nt, tw, tx, a, grid, s);
 }
 
 /* Grouped GEMM over experts: rows [pad_off[e], pad_off[e+1]) of A use W[e*N : (e+1)*N]. */

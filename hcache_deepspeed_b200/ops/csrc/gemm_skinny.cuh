@@ -24,10 +24,12 @@ namespace hds {
 
 constexpr int kSkinnyBF = 128;  // features per CTA (MMA M)
 
-__host__ __device__ constexpr int skinny_stages(int nt) { return nt == 32 ? 5 : 4; }
-__host__ __device__ constexpr int skinny_occupancy(int nt) { return nt == 16 ? 3 : 2; }
-__host__ __device__ constexpr size_t skinny_smem_bytes(int nt) {
-    return static_cast<size_t>(skinny_stages(nt)) * (kSkinnyBF * kGemmBK * 2 + nt * kGemmBK * 2) + 256 + 1024;
+// Grouped (experts): a few hundred units at most, so two CTAs per SM with as many stages as fit keep more bytes in flight than three
+// with four each would when not all of them are there.
+__host__ __device__ constexpr int skinny_stages(int nt, bool grouped = false) { return grouped ? (nt == 64 ? 4 : nt == 32 ? 5 : 6) : nt == 32 ? 5 : 4; }
+__host__ __device__ constexpr int skinny_occupancy(int nt, bool grouped = false) { return nt == 16 && !grouped ? 3 : 2; }
+__host__ __device__ constexpr size_t skinny_smem_bytes(int nt, bool grouped = false) {
+    return static_cast<size_t>(skinny_stages(nt, grouped)) * (kSkinnyBF * kGemmBK * 2 + nt * kGemmBK * 2) + 256 + 1024;
 }
 
 struct SkinnyArgs {
@@ -46,6 +48,8 @@ struct SkinnyArgs {
     const float* w_scale;  // fp8 operands only: per-feature scales [N]
     uint32_t idesc_or;     // fp8 kernels: operand-format bits for 6-bit (E3M2) weights, else 0
     uint32_t w_tx_bytes;   // bytes one weight-tile TMA load reports to the mbarrier (0 = the tile's shared-memory size)
+    const int32_t* group_pad_off;  // kGrouped: expert e owns the rows [pad_off[e], pad_off[e + 1]) of X and of the output (none if empty),
+    int n_groups;                  // the first M of them at most live, and the N weight rows from e * N on
     TpSync sync;           // tensor parallel: the producer acquires the peers' flags before its first activation load
                            // (sync.wait); the last CTA to retire releases the output to the peers (sync.signal)
 };
@@ -107,11 +111,16 @@ __device__ __forceinline__ void skinny_finalize(const SkinnyArgs& a, int n, uint
 // kFp8: both operands are E4M3 codes (a 128-byte row of a tile then holds 128 K-elements instead of 64, i.e. half the
 // weight bytes per MAC); the accumulator is scaled by w_scale[feature] * a_scale[token] right after it leaves TMEM, so
 // split-K partial sums and all three epilogues see real-valued numbers. kBf16 then names the OUTPUT / bias dtype.
-template <int NT, int EPI, bool kBf16, bool kFp8 = false>
-__global__ void __launch_bounds__(kGemmThreads, skinny_occupancy(NT))
+// kGrouped: the experts of a decode step. A unit is (the i-th expert that has rows, feature tile); which experts these are is known
+// to the routing kernels before it only, so nothing is requested ahead of them. Every expert's weights are streamed once: the
+// token-major kernel's 256-wide tiles are too few for that (8 tokens x top 2 of 16 experts of 2048 x 2688: 35 us up and 26 us down,
+// 3.6 TB/s).
+template <int NT, int EPI, bool kBf16, bool kFp8 = false, bool kGrouped = false>
+__global__ void __launch_bounds__(kGemmThreads, skinny_occupancy(NT, kGrouped))
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                   const SkinnyArgs args) {
-    constexpr int STAGES = skinny_stages(NT);
+                   const SkinnyArgs args_in) {
+    SkinnyArgs args = args_in;
+    constexpr int STAGES = skinny_stages(NT, kGrouped);
     constexpr uint32_t W_BYTES = kSkinnyBF * kGemmBK * 2;
     constexpr uint32_t X_BYTES = NT * kGemmBK * 2;
     constexpr uint32_t TMEM_COLS = NT < 32 ? 32 : NT;
@@ -134,7 +143,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int kb_total = (args.K + KB - 1) / KB;
     const int n_t = static_cast<int>(blockIdx.x) % n_tiles;
     const int sp = static_cast<int>(blockIdx.x) / n_tiles;
-    const int kb0 = sp * args.kb_per_split;
+    const int kb0 = kGrouped ? 0 : sp * args.kb_per_split;
     const int kb1 = min(kb_total, kb0 + args.kb_per_split);
     const uint32_t w_tx = args.w_tx_bytes ? args.w_tx_bytes : W_BYTES;
 
@@ -158,6 +167,32 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const uint32_t tmem_base = *tmem_slot;
 
     griddep_launch_dependents();
+    int x_row = 0, w_row = n_t * kSkinnyBF;   // first row of the activations and of the weight tile
+    if constexpr (kGrouped) {
+        // every warp looks for the sp-th expert with rows (kb_per_split covers K: sp is not a split here)
+        griddep_wait();
+        int left = sp, e = -1;
+        for (int e0 = 0; e0 < args.n_groups && e < 0; e0 += 32) {
+            const int i = e0 + static_cast<int>(lane);
+            const bool has = i < args.n_groups && args.group_pad_off[i + 1] > args.group_pad_off[i];
+            const uint32_t m = __ballot_sync(0xffffffffu, has);
+            if (left < __popc(m)) e = e0 + static_cast<int>(__fns(m, 0, left + 1));
+            else left -= __popc(m);
+        }
+        if (e < 0) {      // fewer experts than units: the whole CTA leaves
+            tc_fence_before();
+            __syncthreads();
+            if (warp == 1) {
+                tc_fence_after();
+                tmem_dealloc<TMEM_COLS>(tmem_base);
+            }
+            if (args.sync.signal) tp_signal_tail(args.sync, gridDim.x);
+            return;
+        }
+        x_row = args.group_pad_off[e];
+        w_row += e * args.N;
+        args.out = reinterpret_cast<char*>(args.out) + static_cast<int64_t>(x_row) * args.ldo * 2;
+    }
     if (warp == 0) {
         if (lane == 0) {
             // Weights are never written by a kernel: the first STAGES weight tiles are requested BEFORE waiting for
@@ -166,8 +201,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             const int pre = min(STAGES, kb1 - kb0);
             for (int i = 0; i < pre; ++i) {
                 mbar_expect_tx(&full_bar[i], w_tx + X_BYTES);
-                tma_load_2d(smem_w + i * W_BYTES, &tmap_w, &full_bar[i], (kb0 + i) * KB, n_t * kSkinnyBF,
-                            kEvictFirst);
+                tma_load_2d(smem_w + i * W_BYTES, &tmap_w, &full_bar[i], (kb0 + i) * KB, w_row, kEvictFirst);
             }
             griddep_wait();
             if (args.sync.wait) {  // tensor parallel: the activations were all-gathered into this buffer by the peers
@@ -175,14 +209,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 fence_proxy_async_global();
             }
             for (int i = 0; i < pre; ++i)
-                tma_load_2d(smem_x + i * X_BYTES, &tmap_x, &full_bar[i], (kb0 + i) * KB, 0, kEvictLast);
+                tma_load_2d(smem_x + i * X_BYTES, &tmap_x, &full_bar[i], (kb0 + i) * KB, x_row, kEvictLast);
             uint32_t stage = 0, phase = 1;  // the ring has been filled once
             for (int kb = kb0 + pre; kb < kb1; ++kb) {
                 mbar_wait(&empty_bar[stage], phase ^ 1);
                 mbar_expect_tx(&full_bar[stage], w_tx + X_BYTES);
-                tma_load_2d(smem_x + stage * X_BYTES, &tmap_x, &full_bar[stage], kb * KB, 0, kEvictLast);
-                tma_load_2d(smem_w + stage * W_BYTES, &tmap_w, &full_bar[stage], kb * KB, n_t * kSkinnyBF,
-                            kEvictFirst);
+                tma_load_2d(smem_x + stage * X_BYTES, &tmap_x, &full_bar[stage], kb * KB, x_row, kEvictLast);
+                tma_load_2d(smem_w + stage * W_BYTES, &tmap_w, &full_bar[stage], kb * KB, w_row, kEvictFirst);
                 if (++stage == STAGES) {
                     stage = 0;
                     phase ^= 1;

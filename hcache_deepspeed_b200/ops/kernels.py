@@ -478,6 +478,10 @@ def paged_attention_prefill(q: torch.Tensor, out: torch.Tensor, kv_cache_layer: 
 # ------------------------------------------------------------------------------------------------
 # mixture of experts (ref: ragged_ops/top_k_gating, moe_scatter, moe_gather, cutlass_ops/moe_gemm)
 # ------------------------------------------------------------------------------------------------
+#: most (token, expert) choices of a step whose expert GEMMs stream weights feature-major, 64 rows being the widest token tile
+MOE_FEW = 64
+
+
 def moe_padded_rows(n_tokens: int, n_experts: int, top_k: int) -> int:
     """Row capacity of the scattered activation buffer (each expert's range is padded to 128 rows)."""
     return int(native.cuda_lib().hds_moe_padded_rows(n_tokens, n_experts, top_k))
@@ -512,8 +516,9 @@ def moe_scatter(x: torch.Tensor, xs: torch.Tensor, expert_ids: torch.Tensor, off
 
 
 def moe_gemm(a: torch.Tensor, w_stacked: torch.Tensor, pad_off: torch.Tensor, n_experts: int, out: torch.Tensor,
-             act: int = ACT_IDENTITY, gated: bool = False, limit: float = 0.0) -> torch.Tensor:
-    """Grouped GEMM: rows of ``a`` in expert e's range times ``w_stacked[e*N:(e+1)*N]``ᵀ (``w_stacked``: [E*N, K])."""
+             act: int = ACT_IDENTITY, gated: bool = False, limit: float = 0.0, choices: int = 0) -> torch.Tensor:
+    """Grouped GEMM: rows of ``a`` in expert e's range times ``w_stacked[e*N:(e+1)*N]``ᵀ (``w_stacked``: [E*N, K]). ``choices`` (0: not
+    known): how many rows live in all; up to 64 of them take the kernel that streams the weights (see ``MOE_FEW``)."""
     _check_2d(a, "a")
     _check_2d(out, "out")
     rows, K = a.shape
@@ -523,6 +528,13 @@ def moe_gemm(a: torch.Tensor, w_stacked: torch.Tensor, pad_off: torch.Tensor, n_
         return _gemm_f32(a, w_stacked, out, EPI_GATED if gated else EPI_STORE, act, limit, pad_off, n_experts)
     if act == ACT_SWIGLU_CLAMPED:
         native.check(native.cuda_lib().hds_gemm_next_act_limit(limit), "hds_gemm_next_act_limit")
+    if 0 < choices <= MOE_FEW:
+        rc = native.cuda_lib().hds_moe_gemm_few(_p(a), a.stride(0), _p(w_stacked), w_stacked.stride(0), _p(pad_off), n_experts, choices,
+                                                choices, rows, N, K, _dt(a), EPI_GATED if gated else EPI_STORE, act, _p(out),
+                                                out.stride(0), _stream())
+        native.check(rc, "hds_moe_gemm_few")
+        _count()
+        return out
     rc = native.cuda_lib().hds_moe_gemm(_p(a), a.stride(0), _p(w_stacked), w_stacked.stride(0), _p(pad_off), n_experts, rows,
                                         N, K, _dt(a), EPI_GATED if gated else EPI_STORE, act, _p(out), out.stride(0),
                                         _stream())

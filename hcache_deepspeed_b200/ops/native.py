@@ -97,6 +97,7 @@ def _declare_cuda(lib: ctypes.CDLL, partial: bool = False) -> None:
         "hds_moe_topk_gating": [P, L, I, I, I, I, I, P, F, I, I, P, P, P, P, P],
         "hds_moe_scatter": [P, L, P, L, P, P, P, P, P, I, I, I, I, P, I, P],
         "hds_moe_gemm": [P, L, P, L, P, I, I, I, I, I, I, I, P, L, P],
+        "hds_moe_gemm_few": [P, L, P, L, P, I, I, I, I, I, I, I, I, I, P, L, P],
         "hds_moe_gather": [P, L, P, P, P, L, I, I, I, I, P],
         "hds_gemm_2sm": [P, L, P, L, I, I, I, I, I, I, P, P, L, I, P],
         "hds_quantize_fp8_rows": [P, L, I, I, I, P, L, P, P],

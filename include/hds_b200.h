@@ -311,6 +311,11 @@ int64_t hds_moe_padded_rows(int T, int E, int k);
  * (no bias). max_rows = row capacity of A and out (multiple of 128). */
 int hds_moe_gemm(const void* A, int64_t lda, const void* W_stacked, int64_t ldw, const int32_t* pad_off, int n_experts,
                  int max_rows, int N, int K, int dtype, int epilogue, int act, void* out, int64_t ldo, void* stream);
+/* The same where no expert has more than max_per_expert (<= 64) live rows and at most max_experts have any: the feature-major
+ * kernel streams every weight once. Rows past an expert's live ones may be written, inside its own range. */
+int hds_moe_gemm_few(const void* A, int64_t lda, const void* W_stacked, int64_t ldw, const int32_t* pad_off, int n_experts,
+                     int max_per_expert, int max_experts, int max_rows, int N, int K, int dtype, int epilogue, int act, void* out,
+                     int64_t ldo, void* stream);
 /* out[t, :] += sum_j scores[t, j] * y[mapped_slots[t, j], :]   (out fp32: the pending residual delta) */
 int hds_moe_gather(const void* y, int64_t ldy, const int32_t* mapped_slots, const float* scores, float* out, int64_t ldo,
                    int T, int k, int H, int dtype, void* stream);
