@@ -452,16 +452,23 @@ class RaggedTransformer:
             k = self.ops.k
             E, kk = len(lw.experts), s.top_k
             st = self._moe_state(lw, E, kk)
-            logits = k.gemm(x, lw.w_router, out=st["logits"][:T])
+            logits = k.gemm(x, lw.w_router, out=st["logits"][:T], workspace=self.ws_gemm)
             k.moe_topk_gating(logits, kk, s.norm_topk_prob, st["scores"][:T], st["expert_ids"][:T], st["offsets"][:T],
                               st["counts"])
             rows = k.moe_padded_rows(T, E, kk)
             xs, hs, ys = st["xs"][:rows], st["hs"][:rows], st["ys"][:rows]
             k.moe_scatter(x, xs, st["expert_ids"][:T], st["offsets"][:T], st["counts"], st["pad_off"],
                           st["mapped_slots"][:T], kk)
-            k.moe_gemm(xs, st["w_up"], st["pad_off"], E, hs, act=self.act, gated=s.gated_mlp)
-            k.moe_gemm(hs, st["w_down"], st["pad_off"], E, ys)
-            k.moe_gather(ys, st["mapped_slots"][:T], st["scores"][:T], d32)
+            k.moe_gemm(xs, st["w_up"], st["pad_off"], E, hs, act=self.act, gated=s.gated_mlp, choices=T * kk)
+            k.moe_gemm(hs, st["w_down"], st["pad_off"], E, ys, choices=T * kk)
+            if lw.shared_expert is not None:
+                se = lw.shared_expert
+                act = self.act_buf[:T, :se.w_up.shape[0] // mult]
+                self.ops.gemm(x, se.w_up, act, act=self.act, gated=s.gated_mlp, workspace=self.ws_gemm)
+                shared = self.ops.gemm(act, se.w_down, self.delta16[:T, :s.hidden], workspace=self.ws_gemm)
+                k.moe_gather_shared(ys, st["mapped_slots"][:T], st["scores"][:T], x, lw.w_shared_gate, shared, d32)
+            else:
+                k.moe_gather(ys, st["mapped_slots"][:T], st["scores"][:T], d32)
         else:
             scores = ref.gemm(x, lw.w_router, out_dtype=torch.float32)
             probs = torch.softmax(scores, dim=-1)
@@ -480,7 +487,7 @@ class RaggedTransformer:
                 ye = torch.empty((rows.numel(), s.hidden), dtype=x.dtype, device=x.device)
                 self.ops.gemm(he, ew.w_down, ye)
                 d32.index_add_(0, rows, ye.float() * gate_w[:, None])
-        if lw.shared_expert is not None:
+        if lw.shared_expert is not None and self.device.type != "cuda":
             se = lw.shared_expert
             hs = torch.empty((T, se.w_up.shape[0] // mult), dtype=x.dtype, device=x.device)
             self.ops.gemm(x, se.w_up, hs, act=self.act, gated=s.gated_mlp)

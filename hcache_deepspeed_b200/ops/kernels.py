@@ -642,6 +642,19 @@ def moe_gather(y: torch.Tensor, mapped_slots: torch.Tensor, scores: torch.Tensor
     _count()
 
 
+def moe_gather_shared(y: torch.Tensor, mapped_slots: torch.Tensor, scores: torch.Tensor, x: torch.Tensor, w_gate: torch.Tensor,
+                      ys: torch.Tensor, out: torch.Tensor) -> None:
+    """``moe_gather`` and a shared expert: ``out[t] += ... + sigmoid(x[t] . w_gate) * ys[t]`` (``out`` fp32, ``w_gate`` [1, H])."""
+    T, k = mapped_slots.shape
+    H = y.shape[1]
+    assert out.dtype == torch.float32 and x.dtype == w_gate.dtype == ys.dtype == y.dtype
+    assert x.shape == (T, H) and ys.shape == (T, H) and w_gate.numel() == H and w_gate.is_contiguous()
+    rc = native.cuda_lib().hds_moe_gather_shared(_p(y), y.stride(0), _p(mapped_slots), _p(scores), _p(x), x.stride(0), _p(w_gate), _p(ys),
+                                                 ys.stride(0), _p(out), out.stride(0), T, k, H, _dt(y), _stream())
+    native.check(rc, "hds_moe_gather_shared")
+    _count()
+
+
 # ------------------------------------------------------------------------------------------------
 # expert choice by table, fp32 residual stream, state-space mixers, generic attention
 # ------------------------------------------------------------------------------------------------

@@ -99,6 +99,7 @@ def _declare_cuda(lib: ctypes.CDLL, partial: bool = False) -> None:
         "hds_moe_gemm": [P, L, P, L, P, I, I, I, I, I, I, I, P, L, P],
         "hds_moe_gemm_few": [P, L, P, L, P, I, I, I, I, I, I, I, I, I, P, L, P],
         "hds_moe_gather": [P, L, P, P, P, L, I, I, I, I, P],
+        "hds_moe_gather_shared": [P, L, P, P, P, L, P, P, L, P, L, I, I, I, I, P],
         "hds_gemm_2sm": [P, L, P, L, I, I, I, I, I, I, P, P, L, I, P],
         "hds_quantize_fp8_rows": [P, L, I, I, I, P, L, P, P],
         "hds_gemm_fp8_skinny": [P, L, P, P, L, P, I, I, I, I, I, I, P, P, L, P, L, P, L, I, P],

@@ -319,6 +319,10 @@ int hds_moe_gemm_few(const void* A, int64_t lda, const void* W_stacked, int64_t 
 /* out[t, :] += sum_j scores[t, j] * y[mapped_slots[t, j], :]   (out fp32: the pending residual delta) */
 int hds_moe_gather(const void* y, int64_t ldy, const int32_t* mapped_slots, const float* scores, float* out, int64_t ldo,
                    int T, int k, int H, int dtype, void* stream);
+/* ... + sigmoid(x[t, :] . w_gate) * ys[t, :]: the shared expert's output behind its gate */
+int hds_moe_gather_shared(const void* y, int64_t ldy, const int32_t* mapped_slots, const float* scores, const void* x, int64_t ldx,
+                          const void* w_gate, const void* ys, int64_t ldys, float* out, int64_t ldo, int T, int k, int H, int dtype,
+                          void* stream);
 
 /* ---- FP8 (E4M3) W8A8 GEMM on tcgen05 kind::f8f6f4 ----------------------------------------------------------------
  * hds_quantize_fp8_rows: q[r, :] = e4m3(x[r, :] / scales[r]), scales[r] = amax(x[r, :]) / 448 (per token for

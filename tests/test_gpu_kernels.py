@@ -600,6 +600,50 @@ def test_moe_pipeline(T, E, k, norm):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T,E,k,N,K_,gated", [(1, 3, 1, 128, 64, False), (8, 16, 2, 2688, 2048, False), (16, 5, 1, 200, 328, True), (11, 40, 3, 264, 136, True),
+                                              (16, 70, 4, 136, 512, False)])
+def test_moe_gemm_few(dtype, T, E, k, N, K_, gated):
+    """Experts of a decode step, streamed feature-major: 1..64 choices (token tiles of 16, 32 and 64 rows), experts without rows, more than 32
+    experts, ragged feature tiles and K, against the token-major kernel's own oracle row by row."""
+    torch.manual_seed(T + N)
+    kern = K()
+    x, w = rand(T, K_, dtype=dtype), rand(E * N, K_, dtype=dtype, scale=K_ ** -0.5)
+    ids = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(T)]).int()
+    counts = torch.bincount(ids.flatten().long(), minlength=E)
+    offs = torch.empty_like(ids)
+    seen = [0] * E
+    for t in range(T):
+        for j in range(k):
+            offs[t, j] = seen[int(ids[t, j])]
+            seen[int(ids[t, j])] += 1
+    rows = kern.moe_padded_rows(T, E, k)
+    xs = torch.zeros(rows, K_, dtype=dtype, device="cuda")
+    pad_off, slots = torch.zeros(E + 1, dtype=torch.int32, device="cuda"), torch.empty_like(ids)
+    kern.moe_scatter(x, xs, ids, offs, counts.int(), pad_off, slots, k)
+    out = torch.full((rows, N // 2 if gated else N), 7.0, dtype=dtype, device="cuda")
+    kern.moe_gemm(xs, w, pad_off, E, out, act=3 if gated else 0, gated=gated, choices=T * k)
+    for e in range(E):
+        lo = int(pad_off[e])
+        if counts[e] == 0:
+            continue
+        want = ref.gemm(xs[lo:lo + int(counts[e])], w[e * N:(e + 1) * N], act=3 if gated else 0, gated=gated, out_dtype=torch.float32)
+        torch.testing.assert_close(out[lo:lo + int(counts[e])].float(), want, **tol(dtype))
+    assert bool((out[int(pad_off[E]):] == 7.0).all())      # nothing past the last expert's range
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (5, 2, 2056), (33, 4, 4096)])
+def test_moe_gather_shared(dtype, T, k, H):
+    torch.manual_seed(T + H)
+    x, y, ys, wg = rand(T, H, dtype=dtype), rand(128, H, dtype=dtype), rand(T, H, dtype=dtype), rand(1, H, dtype=dtype, scale=2 * H ** -0.5)
+    slots, scores = torch.randint(0, 128, (T, k), device="cuda", dtype=torch.int32), torch.rand(T, k, device="cuda")
+    out = torch.randn(T, H, device="cuda")
+    want = out.double() + (y.double()[slots.long()] * scores.double()[..., None]).sum(1) + torch.sigmoid(x.double() @ wg.double().T) * ys.double()
+    K().moe_gather_shared(y, slots, scores, x, wg, ys, out)
+    torch.testing.assert_close(out.double(), want, rtol=1e-5, atol=2e-5)      # fp32 sums of up to 4096 products in the gate
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("M,N,K_", [(130, 512, 64), (256, 256, 128), (300, 1000, 2096), (1024, 4096, 1024), (4100, 1376, 512)])
 @pytest.mark.parametrize("bn", [0, 128, 256])
 @pytest.mark.parametrize("mode", ["store", "gated"])
