@@ -115,7 +115,7 @@ def bench_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
             proj, cw, cb, db, a, d, state, ring, spans, single, G, u, dt, y), need)
         mix, w = rnd(rows, inner), torch.ones(inner, device=dev)
         report(f"gated norm {rows}x{inner}", "gated_norm", lambda: K.gated_norm(y, proj[:, :inner], w, mix, G, 1e-5, 0.5), rows * inner * (4 + 2 + 2))
-    from ..ops.backend import latent_splits, pick_packed_splits, windowed_len
+    from ..ops.backend import latent_splits, pick_small_splits, windowed_len
     nq, nkv, D, page = 32, 8, 128, 64
     ws = torch.zeros(256 << 20, dtype=torch.uint8, device=dev)
     for window, keep in ((0, 0), (1024, 0), (1024, 64), (4096, 64)):
@@ -134,10 +134,10 @@ def bench_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
         q, o = rnd(B, nq * D), rnd(B, nq * D)
         items = torch.tensor([[i, i, 1, T - 1] for i in range(B)], dtype=torch.int32, device=dev)
         keys = T if not window else min(T, window + keep)
-        sp = pick_packed_splits(B, nkv, windowed_len(T, window, keep))
-        report(f"attention decode {B}x{T} window {window} keep {keep}", "paged_attention_packed" + ("" if window or keep else " (like)"), lambda:
-               K.paged_attention_prefill(q, o, cache, tables, items, B, nq, nkv, D, page, 0.09, n_splits=sp, workspace=ws, packed=True,
-                                         window=window, keep_first=keep), B * keys * 2 * nkv * D * 2)
+        sp = pick_small_splits(B, nq, nkv, windowed_len(T, window, keep))
+        report(f"attention decode {B}x{T} window {window} keep {keep}", "paged_attention_group" + ("" if window or keep else " (like)"), lambda:
+               K.paged_attention_splitkv(q, o, cache, tables, items, B, nq // nkv, nq, nkv, D, page, sp, 0.09, ws, window=window,
+                                         keep_first=keep, grouped=True), B * keys * 2 * nkv * D * 2)
     del cache
     # gated delta rule: 32 heads of 128 x 128, 16 groups; norm and gate behind it included
     heads, P, N, G = 32, 128, 128, 16
@@ -254,7 +254,7 @@ def bench_lotelix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
     """The same for what Lotelix adds: minGRU, gated linear attention (32 heads of 128 x 128), sinks, sigmoid weights, gates, normed and
     rotated inputs, mixed values, grouped norms, weighted expert inputs."""
     from ..ops import kernels as K
-    from ..ops.backend import pick_packed_splits, windowed_len
+    from ..ops.backend import pick_small_splits, windowed_len
     dev, bf, f32, rnd, report = "cuda", torch.bfloat16, torch.float32, _rnd, _reporter(p, iters, warmup)
     W, T = 4096, PROMPT
     for rows in (T, 64):
@@ -299,10 +299,10 @@ def bench_lotelix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
     items = torch.tensor([[i, i, 1, T - 1] for i in range(B)], dtype=torch.int32, device=dev)
     qd, od, gd = rnd(B, nq * D), rnd(B, nq * D), rnd(B, nq * D)
     for tag, window, opts in cases:
-        sp = pick_packed_splits(B, nkv, windowed_len(T, window))
+        sp = pick_small_splits(B, nq, nkv, windowed_len(T, window))
         opts = dict(opts, gate=gd) if "gate" in opts else opts
-        report(f"attention decode {B}x{T} window {window}", tag, lambda: K.paged_attention_prefill(
-            qd, od, cache, tables, items, B, nq, nkv, D, page, 0.09, n_splits=sp, workspace=ws, packed=True, window=window, **opts),
+        report(f"attention decode {B}x{T} window {window}", tag, lambda: K.paged_attention_splitkv(
+            qd, od, cache, tables, items, B, nq // nkv, nq, nkv, D, page, sp, 0.09, ws, window=window, grouped=True, **opts),
                B * min(T, window or T) * 2 * nkv * D * 2)
     del cache, q, o, gate
     freq, qn, kn, share = torch.ones(64, device=dev), torch.ones(nq * D, device=dev), torch.ones(nkv * D, device=dev), torch.ones(1, device=dev)
@@ -342,7 +342,7 @@ def bench_relulix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
     """The same for what Relulix adds: retention (32 heads of 128 x 128 and of 64 x 128), bounded scores with a one more, rotation with amplitudes,
     queries alone, experts weighed among the chosen, clamped gated experts."""
     from ..ops import kernels as K
-    from ..ops.backend import pick_packed_splits, windowed_len
+    from ..ops.backend import pick_small_splits, windowed_len
     dev, rnd, report = "cuda", _rnd, _reporter(p, iters, warmup)
     W, T, heads, P = 4096, PROMPT, 32, 128
     i32 = lambda *s: torch.zeros(s, dtype=torch.int32, device=dev)  # noqa: E731
@@ -384,13 +384,9 @@ def bench_relulix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
         qd, od = rnd(n, nq * D), rnd(n, nq * D)
         for tag, opts in cases:
             need = n * window * 2 * kvh * D * 2
-            if kvh == nkv:
-                sp = pick_packed_splits(n, kvh, windowed_len(T, window))
-                report(f"attention decode {n}x{T} window {window}, {nq} / {kvh} heads", tag, lambda: K.paged_attention_prefill(
-                    qd, od, cache, tables, items, n, nq, kvh, D, page, 0.09, n_splits=sp, workspace=ws, packed=True, window=window, **opts), need)
-            else:
-                report(f"attention decode {n}x{T} window {window}, {nq} / {kvh} heads", tag, lambda: K.paged_attention_splitkv(
-                    qd, od, cache, tables, items, n, 1, nq, kvh, D, page, 1, 0.09, ws, window=window, **opts), need)
+            sp = pick_small_splits(n, nq, kvh, windowed_len(T, window))
+            report(f"attention decode {n}x{T} window {window}, {nq} / {kvh} heads", tag, lambda: K.paged_attention_splitkv(
+                qd, od, cache, tables, items, n, nq // kvh, nq, kvh, D, page, sp, 0.09, ws, window=window, grouped=nq > kvh, **opts), need)
     del cache
     freq, amp = 1e4**(-torch.arange(64, device=dev) / 64), torch.full((64, ), 1.1, device=dev)
     x, w, b = rnd(T, W), rnd((nq + 2 * nkv) * D, W, scale=0.02), rnd((nq + 2 * nkv) * D)

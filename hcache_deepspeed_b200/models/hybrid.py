@@ -41,8 +41,7 @@ import torch
 
 from ..inference.v2.ragged import RaggedBatchWrapper, RecurrentLayerConfig
 from ..inference.v2.ragged.manager_configs import KVCacheConfig
-from ..ops.backend import (LatentBuffers, latent_launches, pick_decode_splits, pick_packed_splits, pick_prefill_splits, use_packed_decode,
-                           windowed_len)
+from ..ops.backend import LatentBuffers, latent_launches, pick_prefill_splits, pick_small_splits, windowed_len
 from ..ops.kernels import ACT_CODES
 from .arch import (ArchSpec, AttentionSpec, DeltaSpec, FeedForwardSpec, GRUSpec, LatentAttentionSpec, LayerSpec, LinearAttentionSpec, MixerSpec,
                    RetentionSpec, RotationSpec, StateSpaceSpec)
@@ -461,8 +460,7 @@ class HybridTransformer(RaggedTransformer):
                   for l in self.spec.layers if l.mixer.attn is not None}:
             n_q, n_kv, d, window, keep = a
             if batch.n_items_small:
-                pick = pick_packed_splits if use_packed_decode(n_q, n_kv, d) else pick_decode_splits
-                key.append((a, pick(batch.n_items_small, n_kv, windowed_len(batch.max_kv_len_small, window, keep))))
+                key.append((a, pick_small_splits(batch.n_items_small, n_q, n_kv, windowed_len(batch.max_kv_len_small, window, keep))))
             if batch.n_items_large:
                 key.append((a, pick_prefill_splits(batch.n_items_large, n_q, windowed_len(batch.max_kv_len_large, window, keep))))
         if self.dtype != torch.float32:

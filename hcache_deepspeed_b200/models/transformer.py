@@ -27,7 +27,7 @@ import torch
 from ..inference.v2.ragged import DSStateManager, KVCacheConfig, RaggedBatchWrapper
 from ..inference.v2.ragged.manager_configs import DSStateManagerConfig
 from ..ops import reference as ref
-from ..ops.backend import get_ops, pick_decode_splits, pick_packed_splits, use_packed_decode
+from ..ops.backend import get_ops, pick_small_splits
 from ..ops.fp8 import Fp8Weight
 from ..ops.kernels import ACT_CODES
 from .arch import ArchSpec
@@ -208,10 +208,8 @@ class RaggedTransformer:
         if rows is None:
             rows = min(8, max(1, (8 // G) * G))
         worst = 16
-        for n in sorted({1, 2, 4, 8, 16, 32, 64, 128, 256, S}):
-            if n <= S:
-                worst = max(worst, k.splitkv_workspace_bytes(n, n_q, n_kv, d, pick_decode_splits(n, n_kv, 1 << 30), rows))
-        worst = max(worst, k.splitkv_workspace_bytes(S, n_q, n_kv, d, 1, rows))
+        for n in range(1, S + 1):
+            worst = max(worst, k.splitkv_workspace_bytes(n, n_q, n_kv, d, pick_small_splits(n, n_q, n_kv, 1 << 30), rows))
         worst_l = 16
         for n in range(1, 149):
             units = n * n_q
@@ -219,11 +217,6 @@ class RaggedTransformer:
                 break
             sp = min(16, -(-148 // units))
             worst_l = max(worst_l, k.prefill_workspace_bytes(n, n_q, d, sp))
-        if use_packed_decode(n_q, n_kv, d):   # head-packed GQA decode parks its split-KV partials here too
-            for n in range(1, S + 1):
-                sp = pick_packed_splits(n, n_kv, 1 << 30)
-                if sp > 1:
-                    worst_l = max(worst_l, k.prefill_workspace_bytes(n, n_kv, d, sp))
         return worst, worst_l
 
     def _alloc_restore_buffers(self, T: int, S: int, H: int) -> None:
@@ -272,8 +265,7 @@ class RaggedTransformer:
 
     def decode_graph_key(self, batch: RaggedBatchWrapper) -> tuple:
         """Launch geometry of a pure decode step: one CUDA graph serves all steps with the same key."""
-        pick = pick_packed_splits if use_packed_decode(self.n_q, self.n_kv, self.d) else pick_decode_splits
-        return (batch.current_sequences, pick(batch.n_items_small, self.n_kv, batch.max_kv_len_small), batch.rows_per_small_item)
+        return (batch.current_sequences, pick_small_splits(batch.n_items_small, self.n_q, self.n_kv, batch.max_kv_len_small), batch.rows_per_small_item)
 
     def graphable_decode(self, batch: RaggedBatchWrapper) -> bool:
         """May a one-token-per-sequence batch run as a CUDA graph (its launch geometry is what ``decode_graph_key`` says)?"""

@@ -400,15 +400,9 @@ class CudaOps:
         opts = dict(alibi=alibi, window=window, keep_first=keep_first, sink=sink, sigmoid_bias=sigmoid_bias, gate=gate, softcap=softcap)
         if batch.n_items_small:
             n = batch.n_items_small
-            if use_packed_decode(n_q, n_kv, d):
-                # grouped-query decode: the group's query heads share one pass over the KV pages, on the tensor cores
-                splits = pick_packed_splits(n, n_kv, seen(batch.max_kv_len_small))
-                k.paged_attention_prefill(q, out, kv_layer, batch.block_tables(), batch.items_small(), n, n_q, n_kv, d, bs,
-                                          scale, n_splits=splits, workspace=ws_large if splits > 1 else None, packed=True, **opts)
-            else:
-                splits = pick_decode_splits(n, n_kv, seen(batch.max_kv_len_small))
-                k.paged_attention_splitkv(q, out, kv_layer, batch.block_tables(), batch.items_small(), n,
-                                          batch.rows_per_small_item, n_q, n_kv, d, bs, splits, scale, ws_small, **opts)
+            splits = pick_small_splits(n, n_q, n_kv, seen(batch.max_kv_len_small))
+            k.paged_attention_splitkv(q, out, kv_layer, batch.block_tables(), batch.items_small(), n, batch.rows_per_small_item, n_q, n_kv, d,
+                                      bs, splits, scale, ws_small, grouped=n_q > n_kv, **opts)
         if batch.n_items_large:
             n = batch.n_items_large
             splits = pick_prefill_splits(n, n_q, seen(batch.max_kv_len_large))
@@ -608,23 +602,36 @@ def pick_decode_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
     return int(max(1, min(want, cap)))
 
 
-#: grouped-query decode goes to the tensor-core kernel from this group size on (HDS_GQA_PACKED=0 keeps the SIMT kernel)
-PACKED_MIN_GROUP = 4
+def pick_group_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
+    """KV splits of the grouped-query kernel (8 warps and one CTA per SM up to 148 CTAs, else 4 warps and two). Times at head_dim 128:
 
-
-def use_packed_decode(n_q_heads: int, n_kv_heads: int, head_dim: int) -> bool:
-    import os
-    G = n_q_heads // max(1, n_kv_heads)
-    return (head_dim == 128 and G >= PACKED_MIN_GROUP and 128 % G == 0 and os.environ.get("HDS_GQA_PACKED", "1") != "0")
-
-
-def pick_packed_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
-    """KV splits of the head-packed decode kernel (one CTA per SM): as many as keep (items x KV heads x splits) within
-    one wave of CTAs; each split keeps at least 2 tiles of 128 keys."""
+    * up to half as many (item, KV head) pairs as SMs: one wave of CTAs, at least 128 keys (a strip per warp) each. 8 pairs of 16384
+      keys: 132.6 us unsplit, 17.6 in 16; 64 of 4096: 37.6 unsplit, 27.3 in 2; 16 of 1024: 12.1 unsplit, 7.5 in 8. Under 512 keys
+      merging costs what it gains (16 of 300: 6.5 us unsplit, 7.0 in 3).
+    * up to the 296 slots: no split (96 of 700 keys: 10.5 us, 12.6 in 2; 256 of 800: 21.1 us, 26.7 in 2).
+    * beyond: a last wave that is nearly empty costs up to half the rate (320 of 2000 keys: 76.0 us unsplit, 65.1 in 4), so the fewest
+      splits whose waves are 85 % full, of at least 512 keys (320 of 400: 20.8 us unsplit, 28.5 in 4)."""
     ctas = max(1, n_items * n_kv_heads)
-    tiles = max(1, (max_kv_len + 127) // 128)
-    cap = max(1, min(MAX_PREFILL_SPLITS, tiles // 2 if tiles >= 2 else 1))
-    return int(max(1, min(cap, N_SM // ctas)))
+    slots = 2 * N_SM
+    if ctas <= N_SM:
+        cap = max_kv_len // 128 if max_kv_len >= 512 else 1
+        return int(max(1, min(N_SM // ctas, cap, MAX_DECODE_SPLITS)))
+    if ctas <= slots:
+        return 1
+    want, best = 1, 0.0
+    for s in range(1, max(1, min(max_kv_len // 512, 8)) + 1):
+        eff = ctas * s / (slots * -(-ctas * s // slots))
+        if eff >= 0.85:
+            return s
+        if eff > best:
+            want, best = s, eff
+    return want
+
+
+def pick_small_splits(n_items: int, n_q_heads: int, n_kv_heads: int, max_kv_len: int) -> int:
+    """KV splits of a batch's small items, by the kernel that takes them: the one for query heads that share their keys (it reads a key
+    once for the group) or the one for heads of their own."""
+    return (pick_group_splits if n_q_heads > n_kv_heads else pick_decode_splits)(n_items, n_kv_heads, max_kv_len)
 
 
 def pick_prefill_splits(n_items: int, n_q_heads: int, max_kv_len: int) -> int:

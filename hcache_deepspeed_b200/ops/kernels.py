@@ -434,18 +434,18 @@ def paged_attention_splitkv(q: torch.Tensor, out: torch.Tensor, kv_cache_layer: 
                             n_q_heads: int, n_kv_heads: int, head_dim: int, block_size: int, n_splits: int,
                             scale: float, workspace: Optional[torch.Tensor], alibi: Optional[torch.Tensor] = None,
                             window: int = 0, keep_first: int = 0, sink: Optional[torch.Tensor] = None,
-                            sigmoid_bias: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, softcap: float = 0.0) -> None:
+                            sigmoid_bias: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, softcap: float = 0.0,
+                            grouped: bool = False) -> None:
     """kv_cache_layer: [blocks, 2, kvh, bs, d]; items: int32 [n, 4] = (seq, q_row0, n_q, pos0). ``alibi``: fp32 [n_q_heads]
     slopes; score += slope * (key position - query position). ``window``: sliding-window attention, keys (p - window, p] and
     the first ``keep_first`` ones. ``sink``, ``sigmoid_bias`` (fp32 [n_q_heads]) and ``gate`` (rows like ``out``'s): see
-    ``hds_attention_next_sink``."""
+    ``hds_attention_next_sink``. ``grouped``: the kernel for query heads that share their keys (``hds_paged_attention_group``)."""
     lib = native.cuda_lib()
     _arm_alibi(lib, alibi, n_q_heads, window, keep_first, out, sink, sigmoid_bias, gate, softcap)
-    rc = lib.hds_paged_attention_splitkv(_p(q), _p(out), _p(kv_cache_layer), kv_cache_layer.shape[0], _p(block_tables),
-                                         block_tables.stride(0), _p(items), n_items, rows_per_item, n_q_heads,
-                                         n_kv_heads, head_dim, block_size, n_splits, scale, _p(workspace),
-                                         0 if workspace is None else workspace.numel() * workspace.element_size(),
-                                         _dt(q), _stream())
+    fn = lib.hds_paged_attention_group if grouped else lib.hds_paged_attention_splitkv
+    rc = fn(_p(q), _p(out), _p(kv_cache_layer), kv_cache_layer.shape[0], _p(block_tables), block_tables.stride(0), _p(items), n_items,
+            rows_per_item, n_q_heads, n_kv_heads, head_dim, block_size, n_splits, scale, _p(workspace),
+            0 if workspace is None else workspace.numel() * workspace.element_size(), _dt(q), _stream())
     native.check(rc, "hds_paged_attention_splitkv")
     _count()
 

@@ -92,6 +92,7 @@ def _declare_cuda(lib: ctypes.CDLL, partial: bool = False) -> None:
         "hds_cvt_f32": [P, P, L, I, I, P],
         "hds_p2p_gather_rows": [P, P, I, I, I, L, I, P],
         "hds_paged_attention_splitkv": [P, P, P, L, P, I, P, I, I, I, I, I, I, I, F, P, L, I, P],
+        "hds_paged_attention_group": [P, P, P, L, P, I, P, I, I, I, I, I, I, I, F, P, L, I, P],
         "hds_paged_attention_prefill": [P, P, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, I, P],
         "hds_paged_attention_packed": [P, P, P, L, P, I, P, I, I, I, I, I, I, F, I, P, L, I, P],
         "hds_moe_topk_gating": [P, L, I, I, I, I, I, P, F, I, I, P, P, P, P, P],

@@ -204,6 +204,14 @@ int hds_paged_attention_splitkv(const void* q, void* out, const void* kv_cache_l
                                 int block_size, int n_splits, float scale, void* workspace, int64_t workspace_bytes,
                                 int dtype, void* stream);
 
+/* The same for query heads that share their keys (any group size is taken): mma.sync over strips of 16 keys, weights split into
+ * two 16-bit parts; scratch as above. */
+int hds_paged_attention_group(const void* q, void* out, const void* kv_cache_layer, int64_t num_blocks,
+                              const int32_t* block_tables, int max_blocks_per_seq, const hds_attn_item* items,
+                              int n_items, int rows_per_item, int n_q_heads, int n_kv_heads, int head_dim,
+                              int block_size, int n_splits, float scale, void* workspace, int64_t workspace_bytes,
+                              int dtype, void* stream);
+
 /* Split-KV paged attention that allocates nothing and takes no scratch pointer: the partial results and the
  * arrival counters live in a fixed 8 MiB device array that is part of the library image
  * (hds_paged_attention_splitkv_static_capacity() bytes, held by every GPU that loads the library until exit).

@@ -354,6 +354,55 @@ def test_attention_splitkv_decode(dtype, n_q_heads, n_kv, d, bs, n_splits):
         torch.testing.assert_close(out.float(), want.float(), **tol(dtype))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n_q_heads,n_kv,d,bs,n_splits,many", [(8, 1, 128, 16, 1, False), (3, 3, 128, 64, 2, False), (12, 4, 128, 64, 16, False),
+                                                               (2, 2, 64, 32, 9, False), (10, 2, 64, 128, 1, True), (21, 3, 128, 64, 2, True)])
+def test_attention_group_strips(dtype, n_q_heads, n_kv, d, bs, n_splits, many):
+    """Ends of the 16-key strips, fewer strips than warps or splits, every row count of a group, CTAs of eight warps and (``many``: more
+    than 148 of them) of four. Rows behind a sequence's last key are not numbers; outputs keep fp32 weights, so only their own
+    rounding to 16 bits (and the products' order) separates them from 64 bits."""
+    specs = [(c, 1) for c in (0, 14, 15, 16, 30, 31, 47, 63, 64, 127, 500)] * (16 if many else 1) + [(40, 8 // (n_q_heads // n_kv))]
+    q, cache, tables, items = build_paged_problem(specs, n_q_heads, n_kv, d, bs, dtype, seed=5)
+    for (seq, _, n, pos0), t in zip(items, tables.tolist()):
+        if (pos0 + n) % bs:
+            cache[t[(pos0 + n) // bs], :, :, (pos0 + n) % bs:] = float("nan")
+    G, items_t = n_q_heads // n_kv, torch.tensor(items, dtype=torch.int32, device="cuda")
+    rows = max(it[2] for it in items) * G
+    ws = torch.zeros(max(K().splitkv_workspace_bytes(len(items), n_q_heads, n_kv, d, n_splits, rows), 16), dtype=torch.uint8, device="cuda")
+    want, scale = torch.empty_like(q, dtype=torch.float64), 1.0 / math.sqrt(d)
+    for (seq, row, n, pos0), t in zip(items, tables.tolist()):
+        pages = torch.cat([cache[b] for b in t[:(pos0 + n + bs - 1) // bs]], 2).double().repeat_interleave(G, 1)   # [2, heads, keys, d]
+        for i in range(n):
+            k, v = pages[0, :, :pos0 + i + 1], pages[1, :, :pos0 + i + 1]
+            p = torch.softmax((q[row + i].double()[:, None] * k).sum(-1) * scale, -1)
+            want[row + i] = (p[..., None] * v).sum(1)
+    flat = torch.zeros(q.numel() + 1, dtype=dtype, device="cuda")
+    flat[1:] = q.flatten()
+    eps = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
+    for src in (q, flat[1:].view(q.shape)):     # queries on any boundary
+        out = torch.zeros_like(q)
+        K().paged_attention_splitkv(src, out, cache, tables, items_t, len(items), rows, n_q_heads, n_kv, d, bs, n_splits, scale, ws, grouped=True)
+        torch.testing.assert_close(out.double(), want, rtol=eps, atol=2e-5)
+
+
+@pytest.mark.parametrize("opts", ["alibi", "window", "keep", "sink", "sigmoid", "softcap"])
+@pytest.mark.parametrize("n_q_heads,n_kv,d,bs,n_splits", [(16, 4, 128, 64, 1), (6, 2, 64, 128, 3), (8, 1, 128, 16, 12)])
+def test_attention_group_options(opts, n_q_heads, n_kv, d, bs, n_splits):
+    """What may ride on an attention launch, in the grouped kernel as in the one for single heads: windows that begin inside a strip, at
+    its edge and before the first key, kept first tokens on both sides of a strip's end, and the rest with a gate and strided rows."""
+    specs = [(0, 1), (16, 1), (48, 1), (79, 1), (80, 1), (333, 1), (700, 8 // (n_q_heads // n_kv))]
+    q, cache, tables, items = build_paged_problem(specs, n_q_heads, n_kv, d, bs, seed=6)
+    T, items_t = q.shape[0], torch.tensor(items, dtype=torch.int32, device="cuda")
+    vec, gate = torch.linspace(-2.0, 2.0, n_q_heads, device="cuda"), rand(T, n_q_heads * d)
+    kw = {"alibi": dict(alibi=2.0**vec), "window": dict(window=64), "keep": dict(window=33, keep_first=17), "sink": dict(sink=vec, gate=gate, window=200),
+          "sigmoid": dict(sigmoid_bias=vec - 4.0, gate=gate), "softcap": dict(softcap=4.0, sink=vec)}[opts]
+    ws = torch.zeros(K().splitkv_workspace_bytes(len(items), n_q_heads, n_kv, d, n_splits, 8), dtype=torch.uint8, device="cuda")
+    got, want = (torch.zeros(T, n_q_heads * d + 8, dtype=q.dtype, device="cuda")[:, :n_q_heads * d] for _ in range(2))
+    for out, grouped in ((got, True), (want, False)):
+        K().paged_attention_splitkv(q, out, cache, tables, items_t, len(items), 8, n_q_heads, n_kv, d, bs, n_splits, 1 / math.sqrt(d), ws, grouped=grouped, **kw)
+    torch.testing.assert_close(got.float(), want.float(), rtol=2.0**-7, atol=1e-3)     # each rounds its own outputs to bf16
+
+
 def test_attention_splitkv_multirow():
     # short continuations: several query tokens per item (MHA: rows = tokens)
     n_q_heads = n_kv = 4
