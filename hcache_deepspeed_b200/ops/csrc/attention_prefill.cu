@@ -509,6 +509,7 @@ paged_attn_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
 
 }  // namespace hds
 #include "attention_prefill64.cuh"
+#include "attention_pair.cuh"
 namespace hds {
 
 // 64-key tiles, two CTAs per SM (attention_prefill64.cuh): head_dim 128, pages of at most 64 tokens
@@ -534,6 +535,35 @@ static int launch_prefill64(const CUtensorMap& tq, const CUtensorMap& tkv, const
 static bool prefill64_enabled() {
     static const int tile = getenv("HDS_PREFILL_TILE") ? atoi(getenv("HDS_PREFILL_TILE")) : 128;
     return tile == 64;
+}
+
+template <bool kBf16, int kWeights>
+static int launch_pair_as(const CUtensorMap& tq, const CUtensorMap& tkv, const PrefillArgs& a, int n_items, cudaStream_t s) {
+    auto kern = paged_attn_pair_kernel<kBf16, kWeights>;
+    static bool configured[64] = {false};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!configured[dev & 63]) {
+        HDS_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemBytes)));
+        configured[dev & 63] = true;
+    }
+    HDS_CHECK_CUDA(launch_kernel(kern, dim3(n_items, a.n_q_heads / 2), dim3(kPfThreads), kPairSmemBytes, s, tq, tkv, a));
+    return HDS_OK;
+}
+
+template <bool kBf16>
+static int launch_pair(const CUtensorMap& tq, const CUtensorMap& tkv, const PrefillArgs& a, int n_items, cudaStream_t s) {
+    return a.sigmoid_bias != nullptr ? launch_pair_as<kBf16, PF_SIGMOID>(tq, tkv, a, n_items, s)
+           : a.cap_log2 > 0.0f       ? launch_pair_as<kBf16, PF_CAPPED>(tq, tkv, a, n_items, s)
+                                     : launch_pair_as<kBf16, PF_SOFTMAX>(tq, tkv, a, n_items, s);
+}
+
+// Two heads of a group per CTA: head_dim 128, an even group, no ALiBi, no KV split, and at least as many pairs as SMs (at 12 items of
+// 128 tokens x 32 heads, 192 pairs, 28.2 -> 26.9 us; with fewer, one head per CTA keeps more SMs busy).
+static bool use_pair(const PrefillArgs& a, int head_dim, int n_items) {
+    static const int on = getenv("HDS_ATTN_PAIR") ? atoi(getenv("HDS_ATTN_PAIR")) : 1;
+    return on && head_dim == 128 && (a.n_q_heads / a.n_kv_heads) % 2 == 0 && a.alibi == nullptr && a.n_splits == 1 &&
+           static_cast<int64_t>(n_items) * (a.n_q_heads / 2) >= sm_count();
 }
 
 template <int D, bool kBf16, bool kPacked, int kWeights>
@@ -646,6 +676,8 @@ static int attention_tc_impl(bool packed, const void* q, void* out, const void* 
     if (packed)
         return dtype == 0 ? launch_prefill<128, true, true>(tq, tkv, a, n_items, s)
                           : launch_prefill<128, false, true>(tq, tkv, a, n_items, s);
+    if (use_pair(a, head_dim, n_items))
+        return dtype == 0 ? launch_pair<true>(tq, tkv, a, n_items, s) : launch_pair<false>(tq, tkv, a, n_items, s);
     if (head_dim == 128 && block_size <= 64 && alibi == nullptr && window == 0 && out_ld == 0 && opt.sink == nullptr && opt.sigmoid_bias == nullptr &&
         opt.gate == nullptr && opt.softcap == 0.0f && prefill64_enabled())   // none of the options there
         return dtype == 0 ? launch_prefill64<true>(tq, tkv, a, n_items, s) : launch_prefill64<false>(tq, tkv, a, n_items, s);

@@ -597,6 +597,32 @@ def test_attention_prefill_64_key_tiles_subprocess():
     assert " passed" in res.stdout
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("opts", ["plain", "window", "keep", "sink", "sigmoid", "softcap"])
+@pytest.mark.parametrize("n_q_heads,n_kv,bs", [(16, 4, 64), (12, 2, 16), (32, 1, 128)])
+def test_attention_pair(dtype, opts, n_q_heads, n_kv, bs):
+    """Two heads of a group per CTA (from 148 such pairs on): one key tile and many (more than the ring's slots), ragged last tiles, items of
+    one token and of 128, quadrants without rows, windows and kept tokens; against the kernel with one head per CTA, which takes the
+    same items a few at a time."""
+    d = 128
+    specs = [(0, 1), (0, 128), (0, 127), (1, 128), (100, 33), (127, 1), (128, 128), (255, 65), (300, 128), (640, 96), (1000, 128), (1407, 17)] * 3
+    q, cache, tables, items = build_paged_problem(specs, n_q_heads, n_kv, d, bs, dtype, seed=8)
+    T, items_t = q.shape[0], torch.tensor(items, dtype=torch.int32, device="cuda")
+    vec, gate = torch.linspace(-2.0, 2.0, n_q_heads, device="cuda"), rand(T, n_q_heads * d, dtype=dtype)
+    kw = {"plain": {}, "window": dict(window=200), "keep": dict(window=129, keep_first=130), "sink": dict(sink=vec, gate=gate, window=300),
+          "sigmoid": dict(sigmoid_bias=vec - 4.0), "softcap": dict(softcap=4.0, sink=vec)}[opts]
+    got, want = (torch.zeros(T, n_q_heads * d + 8, dtype=dtype, device="cuda")[:, :n_q_heads * d] for _ in range(2))
+    assert len(items) * n_q_heads // 2 >= 148
+    few = max(1, 147 // (n_q_heads // 2))
+    K().paged_attention_prefill(q, got, cache, tables, items_t, len(items), n_q_heads, n_kv, d, bs, 1 / math.sqrt(d), **kw)
+    for i in range(0, len(items), few):
+        part = items_t[i:i + few].contiguous()
+        K().paged_attention_prefill(q, want, cache, tables, part, part.shape[0], n_q_heads, n_kv, d, bs, 1 / math.sqrt(d), **kw)
+    # both round weights to 16 bits, against maxima that may differ by 2^8, and their outputs: the errors of two roundings
+    eps = 2.0**-7 if dtype == torch.bfloat16 else 2.0**-10
+    torch.testing.assert_close(got.float(), want.float(), rtol=2 * eps, atol=eps)
+
+
 # ------------------------------------------------------------------------------------------------
 # mixture of experts
 # ------------------------------------------------------------------------------------------------
