@@ -165,11 +165,7 @@ __global__ void __launch_bounds__(kDtThreads) delta_step_kernel(const DeltaArgs 
     for (int e = threadIdx.x; e < 2 * N + P; e += kDtThreads) {
         const int c = e < N ? inner + g * N + e : e < 2 * N ? inner + a.groups * N + g * N + (e - N) : h * P + (e - 2 * N);
         const float x = load_any<DT>(a.proj, row * a.ld_proj + inner + c);
-        float v = 0.0f;
-        for (int k = 0; k + 1 < taps; ++k) {
-            const int p = pos - (taps - 1) + k;
-            if (p >= 0) v = fmaf(ring[static_cast<int64_t>(p % taps) * C + c], a.conv_w[static_cast<int64_t>(k) * C + c], v);
-        }
+        float v = ssm_earlier_taps(a, ring, c, pos, 0.0f);
         v = fmaf(x, a.conv_w[static_cast<int64_t>(taps - 1) * C + c], v);
         v = ssm_round<DT>(ssm_silu<DT>(v));
         sm[e] = v;

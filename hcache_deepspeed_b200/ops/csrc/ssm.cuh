@@ -51,6 +51,25 @@ __device__ __forceinline__ float ssm_silu(float v) {
 }
 __device__ __forceinline__ float ssm_softplus(float v) { return v > 20.0f ? v : log1pf(expf(v)); }
 
+// The earlier inputs of channel c (from the ring) times their taps, added to v in their order; four inputs' loads are in flight at once.
+__device__ __forceinline__ float ssm_earlier_taps(const SsmArgs& a, const float* ring, int c, int pos, float v) {
+    const int taps = a.taps, C = a.channels();
+    for (int k0 = 0; k0 + 1 < taps; k0 += 4) {
+        float r[4], w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int p = pos - (taps - 1) + k0 + i;
+            const bool ok = k0 + i + 1 < taps && p >= 0;
+            r[i] = ok ? ring[static_cast<int64_t>(p % taps) * C + c] : 0.0f;
+            w[i] = ok ? a.conv_w[static_cast<int64_t>(k0 + i) * C + c] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (k0 + i + 1 < taps && pos - (taps - 1) + k0 + i >= 0) v = fmaf(r[i], w[i], v);
+    }
+    return v;
+}
+
 // Latest inputs of a sequence's convolution channels [c0, c1) -> the ring (all threads of the block).
 template <int DT>
 __device__ __forceinline__ void ssm_save_conv(const SsmArgs& a, const SsmSpan& s, int c0, int c1, int tid, int n_threads) {
