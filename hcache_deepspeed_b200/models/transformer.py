@@ -351,7 +351,12 @@ class RaggedTransformer:
         r0 = min(T, self.tp_rank * per)
         return r0, min(T, r0 + per) - r0
 
-    def _norm(self, x, gamma, out, beta=None, delta=None, res_out=None) -> torch.Tensor:
+    def _fp8_of(self, x: torch.Tensor, w):
+        """Where the norm that writes ``x`` may leave its 8-bit codes for the product with ``w``: nothing (``{}``) unless ``w`` takes them
+        and no rank but this one writes ``x``."""
+        return {"fp8": self.ops.fp8_rows(x)} if isinstance(w, Fp8Weight) and self.tp_size == 1 and x.is_cuda else {}
+
+    def _norm(self, x, gamma, out, beta=None, delta=None, res_out=None, fp8=None) -> torch.Tensor:
         """Norm that folds the pending delta into the residual stream. Under fused tensor parallelism the delta is this
         rank's partial-sum buffer and the kernel performs the collective over NVLink (``hds_norm_tp``): one-shot
         all-reduce for small batches, reduce-scatter + all-gather (``out`` written on every rank, flag signalled, first
@@ -370,7 +375,7 @@ class RaggedTransformer:
             return self.ops.norm(x, gamma, out, beta=beta, delta=delta, res_out=res_out, eps=s.norm_eps,
                                  layer_norm=s.norm == "layer", comm=self.comm, zero_buf=zero_buf, scatter_rows=scatter)
         return self.ops.norm(x, gamma, out, beta=beta, delta=delta, zero_delta=True, res_out=res_out, eps=s.norm_eps,
-                             layer_norm=s.norm == "layer")
+                             layer_norm=s.norm == "layer", **({} if fp8 is None else {"fp8": fp8}))
 
     def _take_tp_wait(self) -> bool:
         """True once after a reduce-scatter + all-gather norm: the caller passes it to the first reader of that output."""
@@ -396,14 +401,14 @@ class RaggedTransformer:
             self._delta_idx = (self._delta_idx + 1) % len(self._delta_bufs)
         return d32
 
-    def _mlp(self, x: torch.Tensor, lw, T: int, force_accum: bool) -> torch.Tensor:
+    def _mlp(self, x: torch.Tensor, lw, T: int, force_accum: bool, fp8=None) -> torch.Tensor:
         s = self.spec
         if s.is_moe:
             return self._moe(x, lw, T)
         n_act = lw.w_up.shape[0] // (2 if s.gated_mlp else 1)
         act = self.act_buf[:T, :n_act]
         self.ops.gemm(x, lw.w_up, act, bias=lw.b_up, act=self.act, gated=s.gated_mlp, workspace=self.ws_gemm,
-                      comm=self.comm, tp_wait=self._take_tp_wait())
+                      comm=self.comm, tp_wait=self._take_tp_wait(), **({} if fp8 is None else {"a_fp8": fp8}))
         return self._row_parallel(act, lw.w_down, lw.b_down, T, force_accum)
 
     def _moe_state(self, lw, E: int, kk: int) -> dict:
@@ -522,12 +527,14 @@ class RaggedTransformer:
         lw = self.w.layers[li]
         T = batch.current_tokens
         kv = self._state_manager
-        self._norm(resid, lw.norm1_g, xn, beta=lw.norm1_b, delta=pending, res_out=resid if pending is not None else None)
+        # (a deferred restore projects this layer's saved rows in between, through the same buffers)
+        codes = self._fp8_of(xn, lw.w_qkv) if self._pending_restore is None else {}
+        self._norm(resid, lw.norm1_g, xn, beta=lw.norm1_b, delta=pending, res_out=resid if pending is not None else None, **codes)
         kv_layer = kv.get_cache(li)
         self._kv_ready(li)
         ops.qkv_rope_kv_append(xn, lw.w_qkv, lw.b_qkv, self.qkv_buf[:T], self.q_buf[:T], kv_layer, batch.tok_pos(), batch.tok_slot(),
                                self.inv_freq, self.n_q, self.n_kv, self.d, s.rot_dim, kv.kv_block_size, workspace=self.ws_gemm,
-                               comm=self.comm, tp_wait=self._take_tp_wait())
+                               comm=self.comm, tp_wait=self._take_tp_wait(), **({"x_fp8": codes["fp8"]} if codes else {}))
         attn = self.attn_buf[:T]
         ops.attention(self.q_buf[:T], attn, kv_layer, batch, self.n_q, self.n_kv, self.d, self.scale,
                       ws_small=self.ws_small, ws_large=self.ws_large, alibi=self.alibi, window=s.window_of(li))
@@ -538,8 +545,9 @@ class RaggedTransformer:
             self._row_parallel(attn, lw.w_o, lw.b_o, T, force_accum=True, last_into_delta=False)
             return self._mlp(xm, lw, T, force_accum=True)
         d1 = self._row_parallel(attn, lw.w_o, lw.b_o, T, force_accum=False)
-        x2 = self._norm(resid, lw.norm2_g, self.xn2[:T], beta=lw.norm2_b, delta=d1, res_out=resid)
-        return self._mlp(x2, lw, T, force_accum=False)
+        codes = self._fp8_of(self.xn2[:T], lw.w_up)
+        x2 = self._norm(resid, lw.norm2_g, self.xn2[:T], beta=lw.norm2_b, delta=d1, res_out=resid, **codes)
+        return self._mlp(x2, lw, T, force_accum=False, **codes)
 
     def _final_hidden(self, resid: torch.Tensor, pending, T: int) -> torch.Tensor:
         """Fold the last pending delta in and apply the final norm."""

@@ -281,8 +281,8 @@ class CudaOps:
         from . import kernels
         self.k = kernels
 
-    def _fp8_act(self, a):
-        """Per-token E4M3 quantisation of ``a`` into persistent buffers (no allocation in steady state)."""
+    def fp8_rows(self, a):
+        """Persistent buffers for the E4M3 codes and scales of ``a``'s rows (no allocation in steady state)."""
         T, K = a.shape
         bufs = self.__dict__.setdefault("_fp8_bufs", {})
         q, s = bufs.get(K, (None, None))
@@ -291,7 +291,11 @@ class CudaOps:
             q = torch.empty(cap, K, dtype=torch.uint8, device=a.device)
             s = torch.empty(cap, dtype=torch.float32, device=a.device)
             bufs[K] = (q, s)
-        return self.k.quantize_fp8_rows(a, q[:T], s[:T])
+        return q[:T], s[:T]
+
+    def _fp8_act(self, a):
+        """Per-token E4M3 quantisation of ``a``."""
+        return self.k.quantize_fp8_rows(a, *self.fp8_rows(a))
 
     def reserve_fp8(self, max_tokens: int, ks, device) -> None:
         """Size the activation-quantisation buffers up front (before any CUDA-graph capture)."""
@@ -300,13 +304,14 @@ class CudaOps:
             bufs[K] = (torch.empty(max_tokens, K, dtype=torch.uint8, device=device),
                        torch.empty(max_tokens, dtype=torch.float32, device=device))
 
-    def gemm(self, a, w, out, bias=None, act=0, gated=False, workspace=None, comm=None, tp_wait=False, tp_signal=False, limit=0.0):
+    def gemm(self, a, w, out, bias=None, act=0, gated=False, workspace=None, comm=None, tp_wait=False, tp_signal=False, limit=0.0, a_fp8=None):
         """``tp_wait``: ``a`` was all-gathered into this GPU's buffer by the peers' norm kernels — the first kernel that
-        reads it acquires their flags. ``tp_signal``: the GEMM's last CTA releases ``out`` to the peers."""
+        reads it acquires their flags. ``tp_signal``: the GEMM's last CTA releases ``out`` to the peers. ``a_fp8``: ``a``'s codes and
+        scales, where the norm has written them."""
         if isinstance(w, Fp8Weight):
             if tp_wait:
                 comm.arm(wait=True)          # consumed by the activation quantiser, the first reader of `a`
-            aq, a_s = self._fp8_act(a)
+            aq, a_s = self._fp8_act(a) if a_fp8 is None else a_fp8
             if tp_signal:
                 comm.arm(signal=True)
             return self.k.gemm_fp8(aq, a_s, w.q, w.scale, out, bias=bias, act=act, gated=gated,
@@ -333,7 +338,7 @@ class CudaOps:
         self.k.gemm_accum(a, w, accum, bias=bias)
 
     def norm(self, x, gamma, out, beta=None, delta=None, zero_delta=False, res_out=None, eps=1e-5, layer_norm=False,
-             comm=None, zero_buf=None, scatter_rows=None):
+             comm=None, zero_buf=None, scatter_rows=None, fp8=None):
         """``comm`` set: ``delta`` is this rank's partial-sum buffer of a row-parallel GEMM (fp32 or 16-bit, symmetric
         memory) and the kernel performs the collective (see ``hds_norm_tp``). ``scatter_rows = (row0, n_rows)`` selects
         the reduce-scatter + all-gather shape: ``out`` (symmetric) is written on every rank and the kernel signals."""
@@ -348,14 +353,14 @@ class CudaOps:
                                   partial_16bit=delta.dtype != torch.float32, zero_buf=zero_buf, beta=beta, res_out=res_out,
                                   eps=eps, layer_norm=layer_norm, wait=not comm.debug_nosync, **kw)
         return self.k.norm(x, gamma, out, beta=beta, delta=delta, zero_delta=zero_delta, res_out=res_out, eps=eps,
-                           layer_norm=layer_norm)
+                           layer_norm=layer_norm, fp8=fp8)
 
     def qkv_rope_kv_append(self, x, w_qkv, b_qkv, qkv_buf, q_out, kv_layer, tok_pos, tok_slot, inv_freq, n_q, n_kv, d,
-                           rot_dim, block_size, workspace=None, comm=None, tp_wait=False):
+                           rot_dim, block_size, workspace=None, comm=None, tp_wait=False, x_fp8=None):
         T = x.shape[0]
         fusable = d in (64, 128) and (inv_freq is None or rot_dim == d)
         if isinstance(w_qkv, Fp8Weight):
-            self.gemm(x, w_qkv, qkv_buf, bias=b_qkv, comm=comm, tp_wait=tp_wait)
+            self.gemm(x, w_qkv, qkv_buf, bias=b_qkv, comm=comm, tp_wait=tp_wait, a_fp8=x_fp8)
             self.k.rope_kv_append(qkv_buf, q_out, kv_layer, tok_pos, tok_slot, inv_freq, n_q, n_kv, d, rot_dim, block_size)
         elif fusable and T >= self.FUSED_QKV_MIN_TOKENS:
             if tp_wait:

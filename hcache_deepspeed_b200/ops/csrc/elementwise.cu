@@ -6,6 +6,7 @@
 //   core_ops/cuda_rms_norm/rms_norm_cuda.cu:18-164, core_ops/cuda_layer_norm/layer_norm_cuda.cu:30-325,
 //   ragged_ops/linear_blocked_kv_rotary/blocked_kv_rotary_cuda.cu:25-194, ragged_ops/embed/embed_cuda.cu:18-80,
 //   ragged_ops/logits_gather/logits_gather_cuda.cu:18-50  (all under deepspeed/inference/v2/kernels/).
+#include "fp8_rows.cuh"
 #include "hds_ptx.cuh"
 #include "hds_host.cuh"
 #include "tp_sync_host.cuh"
@@ -33,12 +34,21 @@ __device__ __forceinline__ float block_sum_256(float v, float* red) {
 //               are cleared after being read so the next accumulating GEMM starts from zero.
 //   res_out   : optional, receives x_in + delta (pre-norm) or the normalised value (post_norm)
 //   out       : normalised output;  row_idx: optional gather of input rows (last-token gather)
-template <int VPT, bool kBf16, bool kLayerNorm, bool kDeltaF32>
+//   kFp8      : the output, as rounded to 16 bits, goes out in E4M3 codes with a scale per row as well, the very ones
+//               hds_quantize_fp8_rows makes of it (a kernel of its own for that took 2.8 us of a 16-token step twice a layer)
+struct NormFp8 {
+    uint8_t* q;
+    int64_t ldq;
+    float* scales;
+};
+template <int VPT, bool kBf16, bool kLayerNorm, bool kDeltaF32, bool kFp8>
 __global__ void __launch_bounds__(kNormThreads)
 norm_kernel(const void* __restrict__ x_in, void* delta, void* res_out, void* __restrict__ out,
             const void* __restrict__ gamma, const void* __restrict__ beta, const int32_t* __restrict__ row_idx,
-            int cols, float eps, int zero_delta, int post_norm, int64_t ld_in, int64_t ld_out) {
+            int cols, float eps, int zero_delta, int post_norm, int64_t ld_in, int64_t ld_out, const NormFp8 f8) {
     __shared__ float red[kNormThreads / 32];
+    uint4 kept[kFp8 ? VPT : 1];
+    float mx = 0.0f;
     pdl_enter();
     const int r_out = blockIdx.x;
     const int r_in = row_idx ? row_idx[r_out] : r_out;
@@ -149,6 +159,28 @@ norm_kernel(const void* __restrict__ x_in, void* delta, void* res_out, void* __r
             const int64_t off = (static_cast<int64_t>(r_out) * ld_out + vi * 8) * 2;
             *reinterpret_cast<uint4*>(reinterpret_cast<char*>(out) + off) = q;
             if (res_out != nullptr && post_norm) *reinterpret_cast<uint4*>(reinterpret_cast<char*>(res_out) + off) = q;
+            if constexpr (kFp8) {
+                kept[i] = q;
+                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) mx = fmaxf(mx, fmaxf(fabsf(unpack_lo<kBf16>(w[j])), fabsf(unpack_hi<kBf16>(w[j]))));
+            }
+        }
+    }
+    if constexpr (kFp8) {
+        mx = warp_max(mx);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+        __syncthreads();
+        mx = red[0];
+#pragma unroll
+        for (int w = 1; w < kNormThreads / 32; ++w) mx = fmaxf(mx, red[w]);
+        const float scale = mx > 0.0f ? mx / kE4M3Max : 1.0f;
+        if (threadIdx.x == 0) f8.scales[r_out] = scale;
+        const float inv = 1.0f / scale;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const int vi = threadIdx.x + i * kNormThreads;
+            if (vi < nvec) *reinterpret_cast<uint2*>(f8.q + static_cast<int64_t>(r_out) * f8.ldq + vi * 8) = e4m3_codes8<kBf16>(kept[i], inv);
         }
     }
 }
@@ -156,12 +188,14 @@ norm_kernel(const void* __restrict__ x_in, void* delta, void* res_out, void* __r
 template <bool kBf16, bool kLayerNorm, bool kDeltaF32>
 static int launch_norm_vpt(int rows, int cols, const void* x, void* delta, void* res_out, void* out, const void* gamma,
                            const void* beta, const int32_t* row_idx, float eps, int zero_delta, int post_norm,
-                           int64_t ld_in, int64_t ld_out, cudaStream_t s) {
+                           int64_t ld_in, int64_t ld_out, const NormFp8& f8, cudaStream_t s) {
     const int nvec = cols / 8;
     const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
 #define HDS_NORM_LAUNCH(V)                                                                                        \
-    launch_kernel(norm_kernel<V, kBf16, kLayerNorm, kDeltaF32>, dim3(rows), dim3(kNormThreads), 0, s, x, delta,    \
-                  res_out, out, gamma, beta, row_idx, cols, eps, zero_delta, post_norm, ld_in, ld_out)
+    (f8.q != nullptr ? launch_kernel(norm_kernel<V, kBf16, kLayerNorm, kDeltaF32, true>, dim3(rows), dim3(kNormThreads), 0, s, x, delta,     \
+                                     res_out, out, gamma, beta, row_idx, cols, eps, zero_delta, post_norm, ld_in, ld_out, f8)           \
+                     : launch_kernel(norm_kernel<V, kBf16, kLayerNorm, kDeltaF32, false>, dim3(rows), dim3(kNormThreads), 0, s, x, delta,    \
+                                     res_out, out, gamma, beta, row_idx, cols, eps, zero_delta, post_norm, ld_in, ld_out, f8))
     if (vpt <= 1) HDS_NORM_LAUNCH(1);
     else if (vpt <= 2) HDS_NORM_LAUNCH(2);
     else if (vpt <= 4) HDS_NORM_LAUNCH(4);
@@ -655,9 +689,18 @@ __global__ void cvt_f32_kernel(float* __restrict__ src, void* __restrict__ dst, 
 
 using namespace hds;
 
+static thread_local hds::NormFp8 g_next_norm_fp8 = {nullptr, 0, nullptr};
+extern "C" int hds_norm_next_fp8(void* q, int64_t ldq, float* scales) {
+    HDS_REQUIRE(q == nullptr || (scales != nullptr && ldq % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 7) == 0), "hds_norm_next_fp8: 8-byte rows and their scales");
+    g_next_norm_fp8 = {static_cast<uint8_t*>(q), ldq, scales};
+    return HDS_OK;
+}
+
 extern "C" int hds_norm(const void* x, int64_t ld_in, void* delta, int delta_is_f32, int zero_delta, void* res_out,
                         void* out, int64_t ld_out, const void* gamma, const void* beta, const int32_t* row_idx,
                         int rows, int cols, float eps, int layer_norm, int post_norm, int dtype, void* stream) {
+    const NormFp8 f8 = g_next_norm_fp8;
+    g_next_norm_fp8 = {nullptr, 0, nullptr};
     HDS_REQUIRE(rows >= 0 && cols > 0 && cols % 8 == 0, "hds_norm: cols must be a positive multiple of 8");
     HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_norm: dtype must be 0 (bf16) or 1 (fp16)");
     HDS_REQUIRE(delta == nullptr || row_idx == nullptr, "hds_norm: delta and row gather are mutually exclusive");
@@ -666,7 +709,7 @@ extern "C" int hds_norm(const void* x, int64_t ld_in, void* delta, int delta_is_
     const bool f32 = delta != nullptr && delta_is_f32;
 #define HDS_NORM_DISPATCH(BF, LN, F32)                                                                            \
     return launch_norm_vpt<BF, LN, F32>(rows, cols, x, delta, res_out, out, gamma, beta, row_idx, eps, zero_delta, \
-                                        post_norm, ld_in, ld_out, s)
+                                        post_norm, ld_in, ld_out, f8, s)
     if (dtype == 0) {
         if (layer_norm) { if (f32) HDS_NORM_DISPATCH(true, true, true); else HDS_NORM_DISPATCH(true, true, false); }
         else            { if (f32) HDS_NORM_DISPATCH(true, false, true); else HDS_NORM_DISPATCH(true, false, false); }

@@ -235,12 +235,17 @@ def qkv_rope_proj(x: torch.Tensor, w_qkv: torch.Tensor, q_out: torch.Tensor, kv_
 def norm(x: torch.Tensor, gamma: torch.Tensor, out: torch.Tensor, *, beta: Optional[torch.Tensor] = None,
          delta: Optional[torch.Tensor] = None, zero_delta: bool = False, res_out: Optional[torch.Tensor] = None,
          row_idx: Optional[torch.Tensor] = None, rows: Optional[int] = None, eps: float = 1e-5,
-         layer_norm: bool = False, post_norm: bool = False) -> torch.Tensor:
+         layer_norm: bool = False, post_norm: bool = False, fp8: Optional[Tuple[torch.Tensor, torch.Tensor]] = None) -> torch.Tensor:
     """RMSNorm / LayerNorm with fused residual add (``delta`` may be the fp32 partial-sum buffer of
-    :func:`gemm_accum`, which is consumed and optionally re-zeroed) and optional row gather."""
+    :func:`gemm_accum`, which is consumed and optionally re-zeroed) and optional row gather. ``fp8``: (codes, scales) that get what
+    :func:`quantize_fp8_rows` would make of ``out``."""
     cols = x.shape[-1]
     n = rows if rows is not None else (row_idx.numel() if row_idx is not None else x.numel() // cols)
     lib = native.cuda_lib()
+    if fp8 is not None:
+        q, scales = fp8
+        assert q.dtype == torch.uint8 and scales.dtype == torch.float32 and q.shape == (n, cols) and scales.numel() >= n and scales.is_contiguous()
+        native.check(lib.hds_norm_next_fp8(_p(q), q.stride(0), _p(scales)), "hds_norm_next_fp8")
     rc = lib.hds_norm(_p(x), x.stride(-2) if x.dim() > 1 else cols, _p(delta),
                       1 if (delta is not None and delta.dtype == torch.float32) else 0, 1 if zero_delta else 0,
                       _p(res_out), _p(out), out.stride(-2) if out.dim() > 1 else cols, _p(gamma), _p(beta), _p(row_idx),

@@ -40,6 +40,7 @@ def _declare_cuda(lib: ctypes.CDLL, partial: bool = False) -> None:
         "hds_restore_kv_proj": [P, L, P, L, I, I, I, P, P, P, P, P, I, I, I, I, P],
         "hds_qkv_rope_proj": [P, L, P, L, I, I, I, P, P, P, P, P, P, P, I, I, I, I, I, P],
         "hds_restore_kv_proj_peers": [P, I, I, L, P, L, I, I, I, P, P, P, P, P, I, I, I, I, P],
+        "hds_norm_next_fp8": [P, L, P],
         "hds_norm": [P, L, P, I, I, P, P, L, P, P, P, I, I, F, I, I, I, P],
         "hds_norm_tp": [I, I, I, P, L, P, P, I, P, P, P, L, P, P, I, I, I, P, P, I, F, I, I, P],
         "hds_fp8_next_weight_format": [I],

@@ -88,6 +88,9 @@ int hds_qkv_rope_proj(const void* x, int64_t ldx, const void* w_qkv, int64_t ldw
 int hds_norm(const void* x, int64_t ld_in, void* delta, int delta_is_f32, int zero_delta, void* res_out, void* out,
              int64_t ld_out, const void* gamma, const void* beta, const int32_t* row_idx, int rows, int cols,
              float eps, int layer_norm, int post_norm, int dtype, void* stream);
+/* The next hds_norm of this host thread also writes its output in E4M3 codes (rows ldq bytes apart, a multiple of 8) and the
+ * rows' scales, as hds_quantize_fp8_rows makes them from `out`. */
+int hds_norm_next_fp8(void* q, int64_t ldq, float* scales);
 
 /* ---- tensor parallelism: this library's own flag protocol over symmetric memory ------------------------------------
  *

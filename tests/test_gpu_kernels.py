@@ -707,6 +707,30 @@ def test_moe_gemm_few(dtype, T, E, k, N, K_, gated):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows,cols,layer", [(1, 8, False), (3, 2056, True), (16, 4096, False), (5, 16384, False)])
+def test_norm_fp8(dtype, rows, cols, layer):
+    """The norm's own 8-bit codes are those of the quantiser, bit for bit, and its 16-bit output is what it is without them; rows of zeros
+    and past the quantiser's registers among them."""
+    torch.manual_seed(rows + cols)
+    x, g, d32 = rand(rows, cols, dtype=dtype), rand(cols, dtype=dtype), torch.randn(rows, cols, device="cuda")
+    x[0], d32[0] = 0.0, 0.0
+    kw = dict(beta=rand(cols, dtype=dtype), layer_norm=True) if layer else {}
+    outs = []
+    for fp8 in (None, (torch.zeros(rows, cols, dtype=torch.uint8, device="cuda"), torch.zeros(rows, device="cuda"))):
+        res, out, delta = torch.empty_like(x), torch.empty_like(x), d32.clone()
+        K().norm(x, g, out, delta=delta, zero_delta=True, res_out=res, fp8=fp8, **kw)
+        outs.append((out, res))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+    q, s = K().quantize_fp8_rows(outs[0][0])
+    assert torch.equal(q, fp8[0]) and torch.equal(s, fp8[1])
+    wide = rand(2, 20000, dtype=dtype)      # longer than a row that stays in registers
+    q, s = K().quantize_fp8_rows(wide)
+    want = (wide.double().abs().amax(1) / 448.0).float()       # (quotients as fp32 rounds them)
+    inv = (1.0 / want.double()).float()
+    assert torch.equal(s, want) and torch.equal(q, (wide.float() * inv[:, None]).to(torch.float8_e4m3fn).view(torch.uint8))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,k,H", [(1, 1, 8), (5, 2, 2056), (33, 4, 4096)])
 def test_moe_gather_shared(dtype, T, k, H):
     torch.manual_seed(T + H)
