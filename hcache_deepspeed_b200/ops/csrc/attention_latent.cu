@@ -19,6 +19,7 @@ namespace hds {
 
 constexpr int kLaThreads = 192, kLaRows = 128, kLaMaxStages = 8, kLaValues = 256;
 constexpr size_t kLaSmemMax = 227 * 1024;
+constexpr int kLaMaxUnits = 148;      // a split launch fills one wave of CTAs at most
 
 struct LatentArgs {
     void* out;                      // [T][heads][rank]
@@ -635,7 +636,8 @@ paged_attn_latent_few_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     }
 }
 
-// Splits of a row meet: CTA = (row tile, row), thread = value of each 128-value block.
+// Splits of a row meet: CTA = (row tile, row), thread = value of each 128-value block. The splits' maxima and sums are read by
+// the threads side by side, and eight splits' values at a time: with a split per key tile there are many.
 template <bool kBf16>
 __global__ void __launch_bounds__(128) latent_merge_kernel(const FewArgs f, int tile_rows) {
     const LatentArgs& a = f.l;
@@ -647,13 +649,17 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const FewArgs f, int 
     const FewTiles ft = fw_tiles(a, item.pos0 + row0 / a.heads, item.pos0 + (row0 + n_rows - 1) / a.heads);
     if (ft.splits == 1) return;       // written by the attention kernel itself
     const int width = f.v_blocks * 128;
+    __shared__ float2 ml_s[kLaMaxUnits];
+    for (int s = threadIdx.x; s < ft.splits; s += 128)
+        ml_s[s] = *reinterpret_cast<const float2*>(a.ws_ml + ((static_cast<int64_t>(unit) * a.n_splits + s) * kLaRows + n) * 2);
+    __syncthreads();
     float mx = -INFINITY, sum = 0.0f;
-    for (int s = 0; s < ft.splits; ++s) mx = fmaxf(mx, a.ws_ml[((static_cast<int64_t>(unit) * a.n_splits + s) * kLaRows + n) * 2]);
+    for (int s = 0; s < ft.splits; ++s) mx = fmaxf(mx, ml_s[s].x);
     float o[5] = {};
-#pragma unroll 4
+#pragma unroll 8
     for (int s = 0; s < ft.splits; ++s) {
         const int64_t slot = static_cast<int64_t>(unit) * a.n_splits + s;
-        const float2 ml = *reinterpret_cast<const float2*>(a.ws_ml + (slot * kLaRows + n) * 2);
+        const float2 ml = ml_s[s];
         const float w = ml.x == -INFINITY ? 0.0f : la_ex2(ml.x - mx);
         sum = fmaf(w, ml.y, sum);
 #pragma unroll
@@ -690,8 +696,6 @@ static size_t la_smem(int panels, int kt, int stages) {
 }
 // keys per tile: 64 when two such tiles fit beside Q, else 32
 static int la_tile(int panels) { return la_smem(panels, 64, 2) <= kLaSmemMax ? 64 : la_smem(panels, 32, 2) <= kLaSmemMax ? 32 : 0; }
-
-constexpr int kLaMaxUnits = 148;      // a split launch fills one wave of CTAs at most
 
 template <bool kBf16, int N>
 static int launch_few(const CUtensorMap& tq, const CUtensorMap& tk, const FewArgs& f, size_t smem, dim3 grid, cudaStream_t s) {

@@ -4,8 +4,8 @@
 //                   the way to the dense q rows, RMS-norms the latent, rotates the shared key part and writes both into the
 //                   token's page row [latent | key part | zeros]. Statistics and angles in fp32.
 //   head_matmul   : out[t][h][n] = sum_k x[t][h][k] w[h][k][n], fp32 accumulation: takes queries to the latent space (and copies
-//                   their rotated part behind), and mean latents to values. One CTA = 16 tokens of one head
-//                   and 64 columns; x is broadcast from shared memory.
+//                   their rotated part behind), and mean latents to values. One CTA = 16 tokens (4 where there are no more) of one
+//                   head and 64 columns; x is broadcast from shared memory.
 #include <type_traits>
 #include "hds_host.cuh"
 #include "hds_ptx.cuh"
@@ -104,12 +104,14 @@ latent_append_kernel(const void* __restrict__ proj, int64_t ld, void* __restrict
     }
 }
 
-constexpr int kHmTok = 16, kHmCols = 64, kHmSlices = 8, kHmBatch = 16, kHmThreads = kHmCols / 2 * kHmSlices;
+constexpr int kHmCols = 64, kHmSlices = 8, kHmThreads = kHmCols / 2 * kHmSlices;
 
 // Warp = one of kHmSlices equal parts of K, lane = two neighbouring columns of the CTA's 64; the parts' sums meet in shared memory.
 // A thread has kHmBatch weights in flight, the first ones before the kernel in front has finished. Tokens of sequences that bring
 // more than `limit` tokens are left alone.
-template <int DT>
+// Up to 4 tokens, tiles of 4: a quarter of the arithmetic (which is all that is left when the weights come early) and registers for all
+// 64 weights of a 512-deep slice. One token of 32 heads, 512 -> 128: 16.9 us with tiles of 16, 4.3 with tiles of 4.
+template <int DT, int kHmTok, int kHmBatch>
 __global__ void __launch_bounds__(kHmThreads)
 head_matmul_kernel(const void* __restrict__ x, int64_t ld_x, int in_width, const void* __restrict__ w, void* __restrict__ out,
                    int64_t ld_out, int out_width, const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ spans, int limit,
@@ -244,21 +246,28 @@ extern "C" int hds_head_matmul(const void* x, int64_t ld_x, int in_width, const 
     HDS_REQUIRE(dtype >= 0 && dtype <= 2, "hds_head_matmul: dtype 0 bf16 / 1 fp16 / 2 fp32");
     HDS_REQUIRE(K >= 1 && N >= 1 && N + copy <= out_width && K + copy <= in_width, "hds_head_matmul: the product fits its rows");
     if (T == 0) return HDS_OK;
-    const size_t smem = (static_cast<size_t>(K) * kHmTok + kHmSlices * kHmTok * kHmCols) * 4;
-    HDS_REQUIRE(smem <= 220 * 1024, "hds_head_matmul: inner size up to 2900");
-    const dim3 grid((T + kHmTok - 1) / kHmTok, heads, (N + kHmCols - 1) / kHmCols), block(kHmThreads);
+    HDS_REQUIRE((static_cast<size_t>(K) * 16 + kHmSlices * 16 * kHmCols) * 4 <= 220 * 1024, "hds_head_matmul: inner size up to 2900");
+    const int tok = T <= 4 ? 4 : 16;
+    const size_t smem = (static_cast<size_t>(K) * tok + kHmSlices * tok * kHmCols) * 4;
+    const dim3 grid((T + tok - 1) / tok, heads, (N + kHmCols - 1) / kHmCols), block(kHmThreads);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define HDS_HM(DT)                                                                                                             \
+#define HDS_HM(DT, TOK, BATCH)                                                                                                 \
     do {                                                                                                                       \
         if (smem > 40 * 1024)                                                                                                  \
-            HDS_CHECK_CUDA(cudaFuncSetAttribute(head_matmul_kernel<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
+            HDS_CHECK_CUDA(cudaFuncSetAttribute(head_matmul_kernel<DT, TOK, BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                                 static_cast<int>(smem)));                                                      \
-        HDS_CHECK_CUDA(launch_kernel(head_matmul_kernel<DT>, grid, block, smem, s, x, ld_x, in_width, w, out, ld_out, out_width, \
-                                     tok_seq, spans, limit, T, K, N, copy));                                                   \
+        HDS_CHECK_CUDA(launch_kernel(head_matmul_kernel<DT, TOK, BATCH>, grid, block, smem, s, x, ld_x, in_width, w, out, ld_out, \
+                                     out_width, tok_seq, spans, limit, T, K, N, copy));                                        \
     } while (0)
-    if (dtype == 0) HDS_HM(0);
-    else if (dtype == 1) HDS_HM(1);
-    else HDS_HM(2);
+    if (tok == 4) {
+        if (dtype == 0) HDS_HM(0, 4, 64);
+        else if (dtype == 1) HDS_HM(1, 4, 64);
+        else HDS_HM(2, 4, 32);
+    } else {
+        if (dtype == 0) HDS_HM(0, 16, 16);
+        else if (dtype == 1) HDS_HM(1, 16, 16);
+        else HDS_HM(2, 16, 16);
+    }
 #undef HDS_HM
     return HDS_OK;
 }

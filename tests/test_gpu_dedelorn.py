@@ -126,6 +126,38 @@ def test_head_matmul_skips_long_sequences(heads, K, N, copy, dtype):
     assert (out[~live] == 7.0).all()
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16, F16])
+@pytest.mark.parametrize("T", [1, 3, 4, 5])
+@pytest.mark.parametrize("heads,K,N,copy", [(3, 17, 29, 6), (4, 512, 128, 0), (2, 600, 40, 0), (5, 96, 512, 32)])
+def test_head_matmul_few_tokens(T, heads, K, N, copy, dtype):
+    """Tiles of 4 tokens and, from 5 on, of 16: a token gets the same sums from both, bit for bit."""
+    iw, ow = K + copy + 3, N + copy + 5
+    x, w = rnd(T, heads * iw, dtype=dtype), rnd(heads, K, N, dtype=dtype, scale=K**-0.5)
+    outs = []
+    for n in (T, T + 16):       # the same tokens in a larger batch
+        out = torch.full((n, heads * ow), 7.0, dtype=dtype, device="cuda")
+        rows = torch.cat([x, x.new_zeros(n - T, heads * iw)])
+        k().head_matmul(rows, w, out, i32(list(range(n))), i32([[i, 1, 0, 0] for i in range(n)]), 8, iw, ow, copy)
+        outs.append(out[:T])
+    assert torch.equal(*outs)
+    x3 = x.float().view(T, heads, iw)
+    want = torch.cat([torch.einsum("thk,hkn->thn", x3[..., :K], w.float()), x3[..., K:K + copy], torch.zeros(T, heads, 5, device="cuda")], -1)
+    tol = 1e-4 if dtype == F32 else 2e-2
+    torch.testing.assert_close(outs[0].float().view(T, heads, ow), want, rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("splits,n_keys", [(33, 4200), (64, 4096), (64, 130), (148, 8300)])
+def test_latent_attention_split_by_tiles(splits, n_keys):
+    """A split per tile of 128 cached rows, more splits than tiles, more than a warp's worth of them, against no split."""
+    heads, rank, width = 32, 512, 576
+    blocks = -(-n_keys // 64)
+    table = torch.randperm(blocks, generator=torch.Generator().manual_seed(1)).to(torch.int32)
+    pages, q = rnd(blocks, 1, 1, 64, width, dtype=BF16), rnd(1, heads, width, seed=2, scale=0.06, dtype=BF16)
+    for window in (0, 1000):
+        want, got = (attend(q, pages, table, n_keys - 1, rank, window, s).float() for s in (1, splits))
+        torch.testing.assert_close(got, want, rtol=1.6e-2, atol=2e-3)       # weights are rounded to bf16 against other maxima
+
+
 # ---- gated delta rule --------------------------------------------------------------------------------------------------
 def delta_case(heads, groups, N, P, taps, T, dtype, seed=0, decay=1.0):
     inner, C = heads * P, heads * P + 2 * groups * N
