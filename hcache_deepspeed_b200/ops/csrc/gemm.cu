@@ -149,7 +149,8 @@ static int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, cons
                                             static_cast<int>(skinny_smem_bytes(NT, kGrouped))));
         configured[dev & 63] = true;
     }
-    HDS_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT, kGrouped), stream, tw, tx, a));
+    HDS_CHECK_CUDA(launch_kernel_cluster(kern, EPI == EPI_RED_F32 || kGrouped ? 1 : a.splits, dim3(grid), dim3(kGemmThreads),
+                                         skinny_smem_bytes(NT, kGrouped), stream, tw, tx, a));
     return HDS_OK;
 }
 
@@ -161,43 +162,16 @@ static int launch_skinny_nt(int nt, const CUtensorMap& tw, const CUtensorMap& tx
     return launch_skinny_inst<64, EPI, kBf16, kGrouped>(tw, tx, a, grid, stream);
 }
 
-// One CTA per (128-feature tile, K split); splits fill the resident slots (SMs x CTAs per SM) once.
+// One CTA per (128-feature tile, K split); splits fill the resident slots (SMs x CTAs per SM) once. No scratch.
 static int launch_skinny(int epi, bool bf16, const void* X, int64_t ldx, const void* W, int64_t ldw, int M, int N,
                          int K, int act, const void* bias, void* out, int64_t ldo, float* accum, int64_t ld_accum,
-                         void* ws, int64_t ws_bytes, int want_splits, cudaStream_t stream) {
+                         int want_splits, cudaStream_t stream) {
     HDS_REQUIRE(M > 0 && N > 0 && K > 0, "gemm: empty problem");
     HDS_REQUIRE(K % 8 == 0 && ldx % 8 == 0 && ldw % 8 == 0, "gemm: K, lda, ldw must be multiples of 8 elements");
     const int nt = skinny_nt(M);
     const int n_tiles = (N + kSkinnyBF - 1) / kSkinnyBF;
     const int kb_total = (K + kGemmBK - 1) / kGemmBK;
-    const int64_t ws_data = (static_cast<int64_t>(n_tiles) * kSkinnyBF * nt * 4 + 255) & ~int64_t(255);
-    const bool can_split = epi == EPI_RED_F32 || (ws != nullptr && ws_bytes >= ws_data + static_cast<int64_t>(n_tiles) * 16);
-    int splits = 1;
-    if (can_split) {
-        if (want_splits > 0) {
-            splits = want_splits;
-        } else {
-            // measured (profiles/kernel_bench_decode_gemm.jsonl, BIG_SHAPES run): fill the resident slots once; past one full
-            // wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4 splits)
-            const int slots = sm_count() * skinny_occupancy(nt);
-            splits = slots / n_tiles;
-            if (n_tiles > slots) {
-                splits = 1;
-                for (int s = 1; s <= 8; ++s) {
-                    const int64_t ctas = static_cast<int64_t>(n_tiles) * s;
-                    const int64_t waves = (ctas + slots - 1) / slots;
-                    if (ctas * 100 >= waves * slots * 80) {
-                        splits = s;
-                        break;
-                    }
-                }
-            }
-            if (splits > kb_total / 4) splits = kb_total / 4;
-            if (splits > 8) splits = 8;
-        }
-        if (splits < 1) splits = 1;
-        if (splits > kb_total) splits = kb_total;
-    }
+    int splits = skinny_splits(n_tiles, kb_total, nt, want_splits, sm_count());
     const int per = (kb_total + splits - 1) / splits;
     splits = (kb_total + per - 1) / per;
     SkinnyArgs a;
@@ -210,10 +184,6 @@ static int launch_skinny(int epi, bool bf16, const void* X, int64_t ldx, const v
     a.out = out; a.ldo = ldo; a.bias = bias;
     a.accum = accum; a.ld_accum = ld_accum;
     a.sync = tp_take_armed();
-    if (splits > 1 && epi != EPI_RED_F32) {
-        a.ws = reinterpret_cast<float*>(ws);
-        a.tickets = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(ws) + ws_data);
-    }
     CUtensorMap tw, tx;
     int rc = make_tmap_2d_16b(&tw, W, static_cast<uint64_t>(K), static_cast<uint64_t>(N),
                               static_cast<uint64_t>(ldw) * 2, kGemmBK, kSkinnyBF, bf16);
@@ -319,8 +289,7 @@ extern "C" int hds_gemm(const void* A, int64_t lda, const void* W, int64_t ldw, 
     // 1.3x faster there, gpurun_out/tp_rank_gemm_probe.jsonl — so the wide-token feature-major form needs N >= 8192)
     if (M <= 64 && ldw >= 0 &&
         (bn == -1 || (bn == 0 && skinny_enabled() && (M <= 16 || (epilogue == EPI_GATED && N >= 8192)))))
-        return launch_skinny(epilogue, dtype == 0, A, lda, W, ldw, M, N, K, act, bias, out, ldo, nullptr, 0, splitk_ws,
-                             splitk_ws_bytes, splits, static_cast<cudaStream_t>(stream));
+        return launch_skinny(epilogue, dtype == 0, A, lda, W, ldw, M, N, K, act, bias, out, ldo, nullptr, 0, splits, static_cast<cudaStream_t>(stream));
     // measured (profiles/kernel_bench_gemm_2sm.txt): with at least one full wave of 256 x 256 pair tiles the
     // cta_group::2 kernel is 1.10-1.20x the single-CTA kernel and level with cuBLAS
     if (bn == 0 && M > 128 && ldw >= 0 && pair_enabled() && lda % 8 == 0 && ldw % 8 == 0 && K % 8 == 0 &&
@@ -370,7 +339,7 @@ extern "C" int hds_gemm_accum(const void* A, int64_t lda, const void* W, int64_t
     HDS_REQUIRE(red_mode >= 0 && red_mode <= 2, "hds_gemm_accum: red_mode 0 (local) / 1 (p2p) / 2 (multicast)");
     if (M <= 64 && ldw >= 0 && red_mode == 0 && n_targets == 1 && (bn == -1 || (bn == 0 && skinny_enabled() && M <= 16)))
         return launch_skinny(EPI_RED_F32, dtype == 0, A, lda, W, ldw, M, N, K, 0, bias, nullptr, 0, accum_ptrs[0],
-                             ld_accum, nullptr, 0, splits, static_cast<cudaStream_t>(stream));
+                             ld_accum, splits, static_cast<cudaStream_t>(stream));
     GemmArgs g;
     memset(&g, 0, sizeof(g));
     Operands ops;

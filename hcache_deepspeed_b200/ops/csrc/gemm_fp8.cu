@@ -368,7 +368,7 @@ static int launch_skinny_fp8_inst(const CUtensorMap& tw, const CUtensorMap& tx, 
                                             static_cast<int>(skinny_smem_bytes(NT))));
         configured[dev & 63] = true;
     }
-    HDS_CHECK_CUDA(launch_kernel(kern, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT), stream, tw, tx, a));
+    HDS_CHECK_CUDA(launch_kernel_cluster(kern, EPI == EPI_RED_F32 ? 1 : a.splits, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT), stream, tw, tx, a));
     return HDS_OK;
 }
 
@@ -402,34 +402,11 @@ extern "C" int hds_gemm_fp8_skinny(const void* Aq, int64_t lda, const float* a_s
     const int nt = M <= 16 ? 16 : M <= 32 ? 32 : 64;
     const int n_tiles = (N + kSkinnyBF - 1) / kSkinnyBF;
     const int kb_total = (K + 127) / 128;
-    const int64_t ws_data = (static_cast<int64_t>(n_tiles) * kSkinnyBF * nt * 4 + 255) & ~int64_t(255);
-    const bool can_split = epilogue == EPI_RED_F32 || (ws != nullptr && ws_bytes >= ws_data + static_cast<int64_t>(n_tiles) * 16);
-    int splits = 1;
-    if (can_split) {
-        if (want_splits > 0) {
-            splits = want_splits;
-        } else {
-            // as launch_skinny (gemm.cu): measured (profiles/kernel_bench_decode_gemm.jsonl, BIG_SHAPES run): fill the resident slots once; past one full
-            // wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4 splits)
-            const int slots = sm_count() * skinny_occupancy(nt);
-            splits = slots / n_tiles;
-            if (n_tiles > slots) {
-                splits = 1;
-                for (int s = 1; s <= 8; ++s) {
-                    const int64_t ctas = static_cast<int64_t>(n_tiles) * s;
-                    const int64_t waves = (ctas + slots - 1) / slots;
-                    if (ctas * 100 >= waves * slots * 80) {
-                        splits = s;
-                        break;
-                    }
-                }
-            }
-            if (splits > kb_total / 4) splits = kb_total / 4;
-            if (splits > 8) splits = 8;
-        }
-        if (splits < 1) splits = 1;
-        if (splits > kb_total) splits = kb_total;
-    }
+    // The splits of a tile need no scratch to meet; but a caller that gives none has always had unsplit sums, and what follows an 8-bit
+    // product rounds to 8 bits again, where a last bit that differs becomes a step of 6 %.
+    const int64_t ws_need = hds_gemm_fp8_skinny_workspace_bytes(M, N);
+    const bool may_split = epilogue == EPI_RED_F32 || (ws != nullptr && ws_bytes >= ws_need);
+    int splits = may_split ? skinny_splits(n_tiles, kb_total, nt, want_splits, sm_count()) : 1;
     const int per = (kb_total + splits - 1) / splits;
     splits = (kb_total + per - 1) / per;
     SkinnyArgs a;
@@ -442,10 +419,6 @@ extern "C" int hds_gemm_fp8_skinny(const void* Aq, int64_t lda, const float* a_s
     a.accum = accum; a.ld_accum = ld_accum;
     a.a_scale = a_scale; a.w_scale = w_scale;
     a.sync = tp_take_armed();
-    if (splits > 1 && epilogue != EPI_RED_F32) {
-        a.ws = reinterpret_cast<float*>(ws);
-        a.tickets = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(ws) + ws_data);
-    }
     CUtensorMap tw, tx;
     const int w_fmt = take_w_fmt();
     HDS_REQUIRE(w_fmt == 0 || K % 128 == 0, "hds_gemm_fp8_skinny: 6-bit weights need K to be a multiple of 128");

@@ -12,8 +12,11 @@
 //   accumulator: TMEM lanes = features, columns = tokens  ->  one epilogue thread owns one output feature
 //
 // Epilogues: store (+bias +act), gated (interleaved gate/up rows of W -> act(g)*u; the partner feature lives
-// in the neighbouring lane), fp32 accumulate into the pending residual delta (split-K needs no tickets there).
-// Split-K for store/gated goes through a feature-major fp32 scratch [N][NT] with one ticket per (tile, warp).
+// in the neighbouring lane), fp32 accumulate into the pending residual delta (split-K needs no meeting there).
+// The K splits of a store / gated tile are a cluster (up to 8): each leaves its sums in its shared memory, behind the cluster's barrier
+// CTA r adds up the tokens r, r + splits, ... of all of them and stores those. Through an fp32 scratch in global memory, with
+// atomic sums and tickets, the end of a tile took 3 - 4 us more: in a decode step of one token, 12288 x 4096 in 4 splits 20.5 us
+// so and 16.5 us now, the gated 22016 x 4096 in 2 splits 31.4 and 27.6 us (6.5 TB/s).
 //
 // Role in the reference: the cuBLAS GEMMs of a decode step (core_ops/blas_kernels/blas.h:31-136) plus the
 // bias / gated activation kernels that follow them.
@@ -32,6 +35,32 @@ __host__ __device__ constexpr size_t skinny_smem_bytes(int nt, bool grouped = fa
     return static_cast<size_t>(skinny_stages(nt, grouped)) * (kSkinnyBF * kGemmBK * 2 + nt * kGemmBK * 2) + 256 + 1024;
 }
 
+// K splits of a decode GEMM of n_tiles feature tiles. Measured (profiles/kernel_bench_decode_gemm.jsonl): fill the resident slots once;
+// past one full wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4
+// splits). At most 8, the size of a portable cluster.
+inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms) {
+    int splits = want;
+    if (want <= 0) {
+        const int slots = sms * skinny_occupancy(nt);
+        splits = slots / n_tiles;
+        if (n_tiles > slots) {
+            splits = 1;
+            for (int s = 1; s <= 8; ++s) {
+                const int64_t ctas = static_cast<int64_t>(n_tiles) * s;
+                const int64_t waves = (ctas + slots - 1) / slots;
+                if (ctas * 100 >= waves * slots * 80) {
+                    splits = s;
+                    break;
+                }
+            }
+        }
+        if (splits > kb_total / 4) splits = kb_total / 4;
+    }
+    if (splits > 8) splits = 8;
+    if (splits > kb_total) splits = kb_total;
+    return splits < 1 ? 1 : splits;
+}
+
 struct SkinnyArgs {
     int M, N, K;
     int splits, kb_per_split;
@@ -42,8 +71,6 @@ struct SkinnyArgs {
     const void* bias;   // [N] I/O dtype, may be null
     float* accum;       // EPI_RED_F32: [M, ld_accum] fp32, accumulated with red.global.add
     int64_t ld_accum;
-    float* ws;          // split-K scratch [N][NT] fp32 (store / gated), zero between calls
-    int32_t* tickets;   // [n_tiles * 4], zero between calls
     const float* a_scale;  // fp8 operands only: per-token scales [M]
     const float* w_scale;  // fp8 operands only: per-feature scales [N]
     uint32_t idesc_or;     // fp8 kernels: operand-format bits for 6-bit (E3M2) weights, else 0
@@ -74,10 +101,10 @@ __device__ __forceinline__ void skinny_tmem_load(uint32_t taddr, float (&v)[NT])
     }
 }
 
-// Final store of one feature column (this thread) for all live tokens. For the gated form the whole warp must call
-// (shuffles): even lanes hold gate features, odd lanes the matching up features.
+// Final store of one feature column (this thread) for the live ones of the tokens t0, t0 + dt, ..., in rows row0 on. For the gated form
+// the whole warp must call (shuffles): even lanes hold gate features, odd lanes the matching up features.
 template <int NT, bool kBf16, bool kGated>
-__device__ __forceinline__ void skinny_finalize(const SkinnyArgs& a, int n, uint32_t lane, float (&v)[NT]) {
+__device__ __forceinline__ void skinny_finalize(const SkinnyArgs& a, int n, uint32_t lane, float (&v)[NT], int t0 = 0, int dt = 1, int row0 = 0) {
     const bool live = n < a.N;
     const float b = (a.bias != nullptr && live) ? load_scalar<kBf16>(a.bias, n) : 0.0f;
 #pragma unroll
@@ -96,16 +123,27 @@ __device__ __forceinline__ void skinny_finalize(const SkinnyArgs& a, int n, uint
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             const float partner = __shfl_xor_sync(0xffffffffu, v[t], 1);
-            if (live && !(lane & 1) && t < a.M)
-                store_scalar<kBf16>(a.out, static_cast<int64_t>(t) * a.ldo + (n >> 1), v[t] * partner);
+            if (live && !(lane & 1) && t0 + t * dt < a.M)
+                store_scalar<kBf16>(a.out, static_cast<int64_t>(row0 + t0 + t * dt) * a.ldo + (n >> 1), v[t] * partner);
         }
     } else {
         if (!live) return;
         apply_act_vec<NT>(v, a.act);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
-            if (t < a.M) store_scalar<kBf16>(a.out, static_cast<int64_t>(t) * a.ldo + n, v[t]);
+            if (t0 + t * dt < a.M) store_scalar<kBf16>(a.out, static_cast<int64_t>(row0 + t0 + t * dt) * a.ldo + n, v[t]);
     }
+}
+
+// a float of CTA `cta` of the cluster, at the place where `p` is in this one
+__device__ __forceinline__ float cluster_load(const float* p, uint32_t cta) {
+    float v;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}\n"
+                 : "=f"(v) : "r"(smem_u32(p)), "r"(cta) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // kFp8: both operands are E4M3 codes (a 128-byte row of a tile then holds 128 K-elements instead of 64, i.e. half the
@@ -118,8 +156,7 @@ __device__ __forceinline__ void skinny_finalize(const SkinnyArgs& a, int n, uint
 template <int NT, int EPI, bool kBf16, bool kFp8 = false, bool kGrouped = false>
 __global__ void __launch_bounds__(kGemmThreads, skinny_occupancy(NT, kGrouped))
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                   const SkinnyArgs args_in) {
-    SkinnyArgs args = args_in;
+                   const SkinnyArgs args) {
     constexpr int STAGES = skinny_stages(NT, kGrouped);
     constexpr uint32_t W_BYTES = kSkinnyBF * kGemmBK * 2;
     constexpr uint32_t X_BYTES = NT * kGemmBK * 2;
@@ -141,8 +178,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const uint32_t lane = lane_id();
     const int n_tiles = (args.N + kSkinnyBF - 1) / kSkinnyBF;
     const int kb_total = (args.K + KB - 1) / KB;
-    const int n_t = static_cast<int>(blockIdx.x) % n_tiles;
-    const int sp = static_cast<int>(blockIdx.x) / n_tiles;
+    // (kGrouped: sp is the place of the expert; else the K split, whose CTAs are neighbours where they are a cluster)
+    const bool meet = EPI != EPI_RED_F32 && !kGrouped && args.splits > 1;
+    const int n_t = meet ? static_cast<int>(blockIdx.x) / args.splits : static_cast<int>(blockIdx.x) % n_tiles;
+    const int sp = meet ? static_cast<int>(blockIdx.x) % args.splits : static_cast<int>(blockIdx.x) / n_tiles;
     const int kb0 = kGrouped ? 0 : sp * args.kb_per_split;
     const int kb1 = min(kb_total, kb0 + args.kb_per_split);
     const uint32_t w_tx = args.w_tx_bytes ? args.w_tx_bytes : W_BYTES;
@@ -191,7 +230,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         }
         x_row = args.group_pad_off[e];
         w_row += e * args.N;
-        args.out = reinterpret_cast<char*>(args.out) + static_cast<int64_t>(x_row) * args.ldo * 2;
     }
     if (warp == 0) {
         if (lane == 0) {
@@ -265,34 +303,35 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         } else {
             constexpr bool kGated = EPI == EPI_GATED;
-            if (args.splits == 1) {
-                skinny_finalize<NT, kBf16, kGated>(args, n, lane, v);
-            } else if (n_t * kSkinnyBF + static_cast<int>(quad * 32) < args.N) {  // warp-uniform
-                float* slot = args.ws + static_cast<int64_t>(n) * NT;
-                if (n < args.N) {
+            if (!meet) {
+                skinny_finalize<NT, kBf16, kGated>(args, n, lane, v, 0, 1, x_row);
+            } else {      // (the stages are free: every product has been read out of them)
+                float* part = reinterpret_cast<float*>(smem) + quad * 32 + lane;
 #pragma unroll
-                    for (int t = 0; t < NT; t += 4) red_add_v4_f32(slot + t, v[t], v[t + 1], v[t + 2], v[t + 3]);
-                }
-                __threadfence();
-                __syncwarp();
-                int last = 0;
-                if (lane == 0) last = (atomicAdd(&args.tickets[n_t * 4 + quad], 1) == args.splits - 1) ? 1 : 0;
-                last = __shfl_sync(0xffffffffu, last, 0);
-                if (last) {
-                    __threadfence();
-                    if (n < args.N) {
+                for (int t = 0; t < NT; ++t)
+                    if (t < args.M) part[t * kSkinnyBF] = v[t];
+            }
+        }
+    }
+    if constexpr (EPI != EPI_RED_F32 && !kGrouped) {
+        if (meet) {
+            __syncwarp();
+            cluster_sync();       // every split's sums are there
+            if (warp >= 2) {
+                constexpr int C = 4;      // tokens at a time
+                const uint32_t quad = warp & 3;
+                const int n = n_t * kSkinnyBF + static_cast<int>(quad * 32 + lane);
+                const float* part = reinterpret_cast<const float*>(smem) + quad * 32 + lane;
+                for (int t0 = sp; t0 < args.M; t0 += C * args.splits) {
+                    float v[C] = {};
+                    for (int s = 0; s < args.splits; ++s)
 #pragma unroll
-                        for (int t = 0; t < NT; t += 4) {
-                            const float4 q = __ldcg(reinterpret_cast<const float4*>(slot + t));
-                            v[t] = q.x; v[t + 1] = q.y; v[t + 2] = q.z; v[t + 3] = q.w;
-                            __stcg(reinterpret_cast<float4*>(slot + t), make_float4(0.f, 0.f, 0.f, 0.f));
-                        }
-                    }
-                    skinny_finalize<NT, kBf16, kGated>(args, n, lane, v);
-                    __syncwarp();
-                    if (lane == 0) args.tickets[n_t * 4 + quad] = 0;
+                        for (int i = 0; i < C; ++i) v[i] += cluster_load(part + min(t0 + i * args.splits, args.M - 1) * kSkinnyBF, s);
+                    skinny_finalize<C, kBf16, EPI == EPI_GATED>(args, n, lane, v, t0, args.splits);
                 }
             }
+            __syncwarp();
+            cluster_sync();       // nobody leaves while its sums are read
         }
     }
 

@@ -313,6 +313,19 @@ def test_qkv_rope_proj(T, n_q, n_kv):
     torch.testing.assert_close(cache.float(), want, **tol(torch.bfloat16))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,K_,splits,gated", [(1, 128, 4096, 8, False), (16, 200, 1024, 3, True), (17, 264, 640, 5, False), (33, 1000, 2048, 7, True), (64, 4096, 512, 2, False),
+                                                 (5, 520, 192, 100, True)])
+def test_gemm_cluster_splits(dtype, M, N, K_, splits, gated):
+    """K splits of a decode GEMM that meet in a cluster: every token tile, more tokens than splits and fewer, ragged features, split counts
+    past what K or a cluster holds; without scratch."""
+    torch.manual_seed(M + N)
+    a, w, b = rand(M, K_, dtype=dtype), rand(N, K_, dtype=dtype, scale=K_ ** -0.5), rand(N, dtype=dtype)
+    out = K().gemm(a, w, bias=b, act=3 if gated else 0, gated=gated, bn=-1, splits=splits)
+    want = ref.gemm(a, w, bias=b, act=3 if gated else 0, gated=gated, out_dtype=torch.float32)
+    torch.testing.assert_close(out.float(), want, **tol(dtype))
+
+
 # ------------------------------------------------------------------------------------------------
 # paged attention
 # ------------------------------------------------------------------------------------------------
