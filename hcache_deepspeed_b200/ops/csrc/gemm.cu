@@ -171,7 +171,7 @@ static int launch_skinny(int epi, bool bf16, const void* X, int64_t ldx, const v
     const int nt = skinny_nt(M);
     const int n_tiles = (N + kSkinnyBF - 1) / kSkinnyBF;
     const int kb_total = (K + kGemmBK - 1) / kGemmBK;
-    int splits = skinny_splits(n_tiles, kb_total, nt, want_splits, sm_count());
+    int splits = skinny_splits(n_tiles, kb_total, nt, want_splits, sm_count(), epi != EPI_RED_F32);
     const int per = (kb_total + splits - 1) / splits;
     splits = (kb_total + per - 1) / per;
     SkinnyArgs a;
@@ -283,12 +283,12 @@ extern "C" int hds_gemm(const void* A, int64_t lda, const void* W, int64_t ldw, 
     HDS_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_GATED, "hds_gemm: epilogue must be 0 (store) or 1 (gated)");
     HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_gemm: dtype must be 0 (bf16) or 1 (fp16)");
     HDS_REQUIRE(epilogue != EPI_GATED || (N % 2 == 0), "hds_gemm: gated epilogue needs an even N");
-    // measured (profiles/kernel_bench.jsonl): the feature-major kernel wins for M <= 16 everywhere and for the gated
-    // MLP-1 up to 64 tokens (1.3-1.5x); plain stores at 32-64 tokens stay on the token-major kernel
-    // (a tensor-parallel rank's MLP-1 is narrow — N = 2752 for Llama-2-7B at TP=8: with 17-64 tokens the token-major kernel is
-    // 1.3x faster there, gpurun_out/tp_rank_gemm_probe.jsonl — so the wide-token feature-major form needs N >= 8192)
+    // Up to 64 tokens the feature-major kernel streams the weights. Plain stores, 64 tokens, token-major against it: 10240 x 8192 40.8
+    // and 32.7 us, 32000 x 8192 90.1 and 83.4, 12288 x 4096 23.5 and 23.3, 6144 x 4096 20.7 and 14.5, 2048 x 2048 9.9 and 7.0; at 17
+    // tokens 40.6 and 29.4, 23.1 and 20.4, 8.2 and 5.3. The gated MLP-1 at 17 - 64 tokens only where it is wide: a tensor-parallel
+    // rank's 2752 features were 1.3 x faster in the token-major kernel.
     if (M <= 64 && ldw >= 0 &&
-        (bn == -1 || (bn == 0 && skinny_enabled() && (M <= 16 || (epilogue == EPI_GATED && N >= 8192)))))
+        (bn == -1 || (bn == 0 && skinny_enabled() && (M <= 16 || epilogue == EPI_STORE || N >= 8192))))
         return launch_skinny(epilogue, dtype == 0, A, lda, W, ldw, M, N, K, act, bias, out, ldo, nullptr, 0, splits, static_cast<cudaStream_t>(stream));
     // measured (profiles/kernel_bench_gemm_2sm.txt): with at least one full wave of 256 x 256 pair tiles the
     // cta_group::2 kernel is 1.10-1.20x the single-CTA kernel and level with cuBLAS
@@ -337,7 +337,10 @@ extern "C" int hds_gemm_accum(const void* A, int64_t lda, const void* W, int64_t
     HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_gemm_accum: dtype must be 0 (bf16) or 1 (fp16)");
     HDS_REQUIRE(n_targets >= 1 && n_targets <= kMaxPeers, "hds_gemm_accum: 1..8 accumulation targets");
     HDS_REQUIRE(red_mode >= 0 && red_mode <= 2, "hds_gemm_accum: red_mode 0 (local) / 1 (p2p) / 2 (multicast)");
-    if (M <= 64 && ldw >= 0 && red_mode == 0 && n_targets == 1 && (bn == -1 || (bn == 0 && skinny_enabled() && M <= 16)))
+    // (as the stores: 64 tokens, token-major against feature-major: 8192 x 28672 79.1 and 73.3 us, 8192 x 8192 25.5 and 23.4, 4096 x 4096
+    // 10.0 and 9.7, 2048 x 2048 6.0 and 5.7; but 1280 x 8192 8.2 and 9.9, and 9.0 and 8.4 at 32 tokens)
+    if (M <= 64 && ldw >= 0 && red_mode == 0 && n_targets == 1 &&
+        (bn == -1 || (bn == 0 && skinny_enabled() && (M <= 32 || N >= 2048))))
         return launch_skinny(EPI_RED_F32, dtype == 0, A, lda, W, ldw, M, N, K, 0, bias, nullptr, 0, accum_ptrs[0],
                              ld_accum, splits, static_cast<cudaStream_t>(stream));
     GemmArgs g;

@@ -406,7 +406,7 @@ extern "C" int hds_gemm_fp8_skinny(const void* Aq, int64_t lda, const float* a_s
     // product rounds to 8 bits again, where a last bit that differs becomes a step of 6 %.
     const int64_t ws_need = hds_gemm_fp8_skinny_workspace_bytes(M, N);
     const bool may_split = epilogue == EPI_RED_F32 || (ws != nullptr && ws_bytes >= ws_need);
-    int splits = may_split ? skinny_splits(n_tiles, kb_total, nt, want_splits, sm_count()) : 1;
+    int splits = may_split ? skinny_splits(n_tiles, kb_total, nt, want_splits, sm_count(), epilogue != EPI_RED_F32) : 1;
     const int per = (kb_total + splits - 1) / splits;
     splits = (kb_total + per - 1) / per;
     SkinnyArgs a;

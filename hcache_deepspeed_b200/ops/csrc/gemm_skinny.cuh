@@ -37,12 +37,15 @@ __host__ __device__ constexpr size_t skinny_smem_bytes(int nt, bool grouped = fa
 
 // K splits of a decode GEMM of n_tiles feature tiles. Measured (profiles/kernel_bench_decode_gemm.jsonl): fill the resident slots once;
 // past one full wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4
-// splits). At most 8, the size of a portable cluster.
-inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms) {
+// splits). At most 8, the size of a portable cluster. A cluster needs its slots in one GPC, so that some stay empty: where the splits
+// meet in one, they fill no more than 87 % (96 tiles x 3 of 296 slots: 27.7 us at 17 tokens of 12288 x 4096, 20.4 us in 2).
+inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms, bool clusters) {
     int splits = want;
     if (want <= 0) {
         const int slots = sms * skinny_occupancy(nt);
         splits = slots / n_tiles;
+        if (clusters && n_tiles <= slots)
+            while (splits > 1 && static_cast<int64_t>(n_tiles) * (splits < 8 ? splits : 8) * 100 > static_cast<int64_t>(slots) * 87) --splits;
         if (n_tiles > slots) {
             splits = 1;
             for (int s = 1; s <= 8; ++s) {
