@@ -403,16 +403,24 @@ class CudaOps:
         # with a sliding window an item reads at most window + one tile of keys: size the KV split for that
         seen = lambda n_kv_tokens: windowed_len(n_kv_tokens, window, keep_first)  # noqa: E731
         opts = dict(alibi=alibi, window=window, keep_first=keep_first, sink=sink, sigmoid_bias=sigmoid_bias, gate=gate, softcap=softcap)
+
+        def by_head(items, n, max_kv_len):
+            splits = pick_prefill_splits(n, n_q, seen(max_kv_len))
+            k.paged_attention_prefill(q, out, kv_layer, batch.block_tables(), items, n, n_q, n_kv, d, bs, scale, n_splits=splits,
+                                      workspace=ws_large if splits > 1 else None, **opts)
+
         if batch.n_items_small:
             n = batch.n_items_small
-            splits = pick_small_splits(n, n_q, n_kv, seen(batch.max_kv_len_small))
-            k.paged_attention_splitkv(q, out, kv_layer, batch.block_tables(), batch.items_small(), n, batch.rows_per_small_item, n_q, n_kv, d,
-                                      bs, splits, scale, ws_small, grouped=n_q > n_kv, **opts)
+            # the batch may have been built for smaller groups than this attention's: its items then hold more query rows
+            rows = max(batch.rows_per_small_item, batch.rows_per_small_item // batch.group * (n_q // n_kv))
+            if rows > MAX_SMALL_ROWS:
+                by_head(batch.items_small(), n, batch.max_kv_len_small)
+            else:
+                splits = pick_small_splits(n, n_q, n_kv, seen(batch.max_kv_len_small))
+                k.paged_attention_splitkv(q, out, kv_layer, batch.block_tables(), batch.items_small(), n, rows, n_q, n_kv, d, bs, splits, scale,
+                                          ws_small, grouped=n_q > n_kv, **opts)
         if batch.n_items_large:
-            n = batch.n_items_large
-            splits = pick_prefill_splits(n, n_q, seen(batch.max_kv_len_large))
-            k.paged_attention_prefill(q, out, kv_layer, batch.block_tables(), batch.items_large(), n, n_q, n_kv, d, bs,
-                                      scale, n_splits=splits, workspace=ws_large if splits > 1 else None, **opts)
+            by_head(batch.items_large(), batch.n_items_large, batch.max_kv_len_large)
 
     # ---- stacks of unlike layers ----------------------------------------------------------------------
     def embed_f32(self, ids, weight, out, **kw):
@@ -580,6 +588,7 @@ N_SM = 148
 MAX_DECODE_SPLITS = 16
 MAX_PREFILL_SPLITS = 16
 MAX_LATENT_SPLITS = 64
+MAX_SMALL_ROWS = 8      # query rows per item and KV head that the kernels of few rows take
 
 
 def pick_decode_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:

@@ -1,0 +1,68 @@
+"""Which kernel a batch's attention goes to, and with what arguments: the launches of ``CudaOps.attention`` recorded on the CPU."""
+import types
+
+import pytest
+import torch
+
+from hcache_deepspeed_b200.inference.v2.ragged import DSStateManager, KVCacheConfig, RaggedBatchWrapper
+from hcache_deepspeed_b200.inference.v2.ragged.manager_configs import DSStateManagerConfig
+from hcache_deepspeed_b200.ops.backend import CudaOps
+
+
+class Recorder:
+    """Stands in for the kernel bindings: notes every call's name and arguments."""
+
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        return lambda *a, **kw: self.calls.append((name, a, kw))
+
+
+def batch_of(specs, group, block=64):
+    """A ragged batch of (seen, new) sequences, built for query groups of ``group``."""
+    blocks = sum(-(-(s + n) // block) for s, n in specs) + 1
+    cfg = DSStateManagerConfig(max_tracked_sequences=len(specs), max_ragged_batch_size=max(512, len(specs)), max_ragged_sequence_count=len(specs),
+                               max_context=max(s + n for s, n in specs) + block, memory_config={"mode": "allocate", "size": blocks * block * 2 * 8 * 4})
+    m = DSStateManager(cfg, (KVCacheConfig(block_size=block, cache_shape=(1, 1, 8), cache_dtype="fp32",
+                                           max_blocks_per_allocation_group=-(-cfg.max_context // block)), ), device=torch.device("cpu"))
+    b = RaggedBatchWrapper(cfg, block_size=block, group=group, device=torch.device("cpu"))
+    for uid, (seen, new) in enumerate(specs):
+        s = m.get_or_create_sequence(uid)
+        s.extend_kv_cache(m.allocate_blocks(-(-(seen + new) // block)))
+        s._seen_tokens = seen
+        s.pre_forward(new)
+        b.insert_sequence(s, torch.zeros(new, dtype=torch.int64))
+    b.finalize()
+    return b
+
+
+def launches(batch, n_q, n_kv, d=128, dtype=torch.bfloat16, **kw):
+    ops = object.__new__(CudaOps)
+    ops.k = Recorder()
+    q = torch.zeros(batch.current_tokens, n_q * d, dtype=dtype)
+    ops.attention(q, torch.zeros_like(q), torch.zeros(1), batch, n_q, n_kv, d, 1.0, **kw)
+    out = []
+    for name, a, kw in ops.k.calls:
+        c = types.SimpleNamespace(name=name, n_items=a[5], grouped=kw.get("grouped", False))
+        if name == "paged_attention_splitkv":
+            c.rows, c.splits, c.workspace = a[6], a[11], a[13]
+        else:
+            c.rows, c.splits, c.workspace = None, kw["n_splits"], kw["workspace"]
+        out.append(c)
+    return out
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(4, 4), (4, 2), (6, 2), (8, 2), (16, 2), (32, 2)])
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+def test_rows_of_small_items(n_q, n_kv, group):
+    """A batch may have been built for other groups than the attention has (a wrapper's default is 1): the kernels of few rows get
+    no more than their 8, and are told of all of them; other items go to the kernel that takes 128 tokens of a head."""
+    for new in range(1, 9):
+        b = batch_of([(100, new), (30, 1)], group)
+        calls = launches(b, n_q, n_kv)
+        assert sum(c.n_items for c in calls) == 2
+        for c in calls:
+            if c.name == "paged_attention_splitkv":
+                tokens = max(it[2] for it in b.items_small().tolist())
+                assert tokens * (n_q // n_kv) <= c.rows <= 8

@@ -416,6 +416,21 @@ def test_attention_group_options(opts, n_q_heads, n_kv, d, bs, n_splits):
     torch.testing.assert_close(got.float(), want.float(), rtol=2.0**-7, atol=1e-3)     # each rounds its own outputs to bf16
 
 
+@pytest.mark.parametrize("n_q_heads,n_kv,d", [(8, 2, 128), (6, 2, 128), (4, 2, 64)])
+def test_attention_of_a_batch_for_smaller_groups(n_q_heads, n_kv, d):
+    """Items of up to 8 tokens, as a batch built for heads of their own has them, under grouped attention: every row is computed."""
+    import types
+    from hcache_deepspeed_b200.ops.backend import CudaOps
+    q, cache, tables, items = build_paged_problem([(40, 8), (300, 3), (17, 1)], n_q_heads, n_kv, d, 64, seed=9)
+    items_t = torch.tensor(items, dtype=torch.int32, device="cuda")
+    batch = types.SimpleNamespace(block_size=64, group=1, n_items_small=3, n_items_large=0, rows_per_small_item=8, max_kv_len_small=303,
+                                  block_tables=lambda: tables, items_small=lambda: items_t)
+    out = torch.full_like(q, float("nan"))
+    CudaOps().attention(q.view(q.shape[0], -1), out.view(q.shape[0], -1), cache, batch, n_q_heads, n_kv, d, 1 / math.sqrt(d))
+    want = ref.paged_attention(q, cache, tables, items, n_q_heads, n_kv, 1 / math.sqrt(d))
+    torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
+
+
 def test_attention_splitkv_multirow():
     # short continuations: several query tokens per item (MHA: rows = tokens)
     n_q_heads = n_kv = 4
