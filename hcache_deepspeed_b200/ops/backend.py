@@ -405,7 +405,7 @@ class CudaOps:
         opts = dict(alibi=alibi, window=window, keep_first=keep_first, sink=sink, sigmoid_bias=sigmoid_bias, gate=gate, softcap=softcap)
 
         def by_head(items, n, max_kv_len):
-            splits = pick_prefill_splits(n, n_q, seen(max_kv_len))
+            splits = pick_prefill_splits(n, n_q, seen(max_kv_len)) if ws_large is not None else 1
             k.paged_attention_prefill(q, out, kv_layer, batch.block_tables(), items, n, n_q, n_kv, d, bs, scale, n_splits=splits,
                                       workspace=ws_large if splits > 1 else None, **opts)
 
@@ -416,7 +416,7 @@ class CudaOps:
             if rows > MAX_SMALL_ROWS:
                 by_head(batch.items_small(), n, batch.max_kv_len_small)
             else:
-                splits = pick_small_splits(n, n_q, n_kv, seen(batch.max_kv_len_small))
+                splits = pick_small_splits(n, n_q, n_kv, seen(batch.max_kv_len_small)) if ws_small is not None else 1
                 k.paged_attention_splitkv(q, out, kv_layer, batch.block_tables(), batch.items_small(), n, rows, n_q, n_kv, d, bs, splits, scale,
                                           ws_small, grouped=n_q > n_kv, **opts)
         if batch.n_items_large:

@@ -66,3 +66,13 @@ def test_rows_of_small_items(n_q, n_kv, group):
             if c.name == "paged_attention_splitkv":
                 tokens = max(it[2] for it in b.items_small().tolist())
                 assert tokens * (n_q // n_kv) <= c.rows <= 8
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(32, 32), (32, 8), (64, 8)])
+@pytest.mark.parametrize("seqs,seen", [(40, 2000), (2, 700), (40, 100)])
+def test_no_scratch_no_split(n_q, n_kv, seqs, seen):
+    """Callers without scratch (the module and kernel wrappers) get unsplit launches, whatever the batch."""
+    b = batch_of([(seen, 1)] * seqs, n_q // n_kv)
+    assert [c.splits for c in launches(b, n_q, n_kv)] == [1]
+    if seqs == 2:
+        assert launches(b, n_q, n_kv, ws_small=torch.zeros(1), ws_large=torch.zeros(1))[0].splits > 1
