@@ -134,7 +134,7 @@ def bench_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
         q, o = rnd(B, nq * D), rnd(B, nq * D)
         items = torch.tensor([[i, i, 1, T - 1] for i in range(B)], dtype=torch.int32, device=dev)
         keys = T if not window else min(T, window + keep)
-        sp = pick_small_splits(B, nq, nkv, windowed_len(T, window, keep))
+        sp = pick_small_splits(B, nq, nkv, D, windowed_len(T, window, keep))
         report(f"attention decode {B}x{T} window {window} keep {keep}", "paged_attention_group" + ("" if window or keep else " (like)"), lambda:
                K.paged_attention_splitkv(q, o, cache, tables, items, B, nq // nkv, nq, nkv, D, page, sp, 0.09, ws, window=window,
                                          keep_first=keep, grouped=True), B * keys * 2 * nkv * D * 2)
@@ -299,7 +299,7 @@ def bench_lotelix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
     items = torch.tensor([[i, i, 1, T - 1] for i in range(B)], dtype=torch.int32, device=dev)
     qd, od, gd = rnd(B, nq * D), rnd(B, nq * D), rnd(B, nq * D)
     for tag, window, opts in cases:
-        sp = pick_small_splits(B, nq, nkv, windowed_len(T, window))
+        sp = pick_small_splits(B, nq, nkv, D, windowed_len(T, window))
         opts = dict(opts, gate=gd) if "gate" in opts else opts
         report(f"attention decode {B}x{T} window {window}", tag, lambda: K.paged_attention_splitkv(
             qd, od, cache, tables, items, B, nq // nkv, nq, nkv, D, page, sp, 0.09, ws, window=window, grouped=True, **opts),
@@ -342,7 +342,7 @@ def bench_relulix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
     """The same for what Relulix adds: retention (32 heads of 128 x 128 and of 64 x 128), bounded scores with a one more, rotation with amplitudes,
     queries alone, experts weighed among the chosen, clamped gated experts."""
     from ..ops import kernels as K
-    from ..ops.backend import pick_small_splits, windowed_len
+    from ..ops.backend import pick_small_splits, use_grouped_decode, windowed_len
     dev, rnd, report = "cuda", _rnd, _reporter(p, iters, warmup)
     W, T, heads, P = 4096, PROMPT, 32, 128
     i32 = lambda *s: torch.zeros(s, dtype=torch.int32, device=dev)  # noqa: E731
@@ -384,9 +384,9 @@ def bench_relulix_kernels(p: Dict[str, float], iters: int, warmup: int) -> None:
         qd, od = rnd(n, nq * D), rnd(n, nq * D)
         for tag, opts in cases:
             need = n * window * 2 * kvh * D * 2
-            sp = pick_small_splits(n, nq, kvh, windowed_len(T, window))
+            sp = pick_small_splits(n, nq, kvh, D, windowed_len(T, window))
             report(f"attention decode {n}x{T} window {window}, {nq} / {kvh} heads", tag, lambda: K.paged_attention_splitkv(
-                qd, od, cache, tables, items, n, nq // kvh, nq, kvh, D, page, sp, 0.09, ws, window=window, grouped=nq > kvh, **opts), need)
+                qd, od, cache, tables, items, n, nq // kvh, nq, kvh, D, page, sp, 0.09, ws, window=window, grouped=use_grouped_decode(nq, kvh, D), **opts), need)
     del cache
     freq, amp = 1e4**(-torch.arange(64, device=dev) / 64), torch.full((64, ), 1.1, device=dev)
     x, w, b = rnd(T, W), rnd((nq + 2 * nkv) * D, W, scale=0.02), rnd((nq + 2 * nkv) * D)

@@ -460,7 +460,7 @@ class HybridTransformer(RaggedTransformer):
                   for l in self.spec.layers if l.mixer.attn is not None}:
             n_q, n_kv, d, window, keep = a
             if batch.n_items_small:
-                key.append((a, pick_small_splits(batch.n_items_small, n_q, n_kv, windowed_len(batch.max_kv_len_small, window, keep))))
+                key.append((a, pick_small_splits(batch.n_items_small, n_q, n_kv, d, windowed_len(batch.max_kv_len_small, window, keep))))
             if batch.n_items_large:
                 key.append((a, pick_prefill_splits(batch.n_items_large, n_q, windowed_len(batch.max_kv_len_large, window, keep))))
         if self.dtype != torch.float32:

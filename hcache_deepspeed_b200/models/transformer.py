@@ -209,7 +209,7 @@ class RaggedTransformer:
             rows = min(8, max(1, (8 // G) * G))
         worst = 16
         for n in range(1, S + 1):
-            worst = max(worst, k.splitkv_workspace_bytes(n, n_q, n_kv, d, pick_small_splits(n, n_q, n_kv, 1 << 30), rows))
+            worst = max(worst, k.splitkv_workspace_bytes(n, n_q, n_kv, d, pick_small_splits(n, n_q, n_kv, d, 1 << 30), rows))
         worst_l = 16
         for n in range(1, 149):
             units = n * n_q
@@ -265,7 +265,8 @@ class RaggedTransformer:
 
     def decode_graph_key(self, batch: RaggedBatchWrapper) -> tuple:
         """Launch geometry of a pure decode step: one CUDA graph serves all steps with the same key."""
-        return (batch.current_sequences, pick_small_splits(batch.n_items_small, self.n_q, self.n_kv, batch.max_kv_len_small), batch.rows_per_small_item)
+        splits = pick_small_splits(batch.n_items_small, self.n_q, self.n_kv, self.d, batch.max_kv_len_small)
+        return (batch.current_sequences, splits, batch.rows_per_small_item)
 
     def graphable_decode(self, batch: RaggedBatchWrapper) -> bool:
         """May a one-token-per-sequence batch run as a CUDA graph (its launch geometry is what ``decode_graph_key`` says)?"""

@@ -416,9 +416,9 @@ class CudaOps:
             if rows > MAX_SMALL_ROWS:
                 by_head(batch.items_small(), n, batch.max_kv_len_small)
             else:
-                splits = pick_small_splits(n, n_q, n_kv, seen(batch.max_kv_len_small)) if ws_small is not None else 1
+                splits = pick_small_splits(n, n_q, n_kv, d, seen(batch.max_kv_len_small)) if ws_small is not None else 1
                 k.paged_attention_splitkv(q, out, kv_layer, batch.block_tables(), batch.items_small(), n, rows, n_q, n_kv, d, bs, splits, scale,
-                                          ws_small, grouped=n_q > n_kv, **opts)
+                                          ws_small, grouped=use_grouped_decode(n_q, n_kv, d), **opts)
         if batch.n_items_large:
             by_head(batch.items_large(), batch.n_items_large, batch.max_kv_len_large)
 
@@ -617,6 +617,14 @@ def pick_decode_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
     return int(max(1, min(want, cap)))
 
 
+def use_grouped_decode(n_q_heads: int, n_kv_heads: int, head_dim: int) -> bool:
+    """Whether a batch's small items go to the grouped-query kernel (HDS_GQA_PACKED=0: none). It keeps a weight in two 16-bit parts, so it
+    takes the groups whose decode kernel rounded weights to 16 bits: 4 and 8 heads at 128 dims (64 x 250 keys of 8 KV heads with 8
+    heads each: 34.4 us there, 19.7 here). All others stay with the split-KV kernel, whose weights are fp32."""
+    import os
+    return head_dim == 128 and n_q_heads // max(1, n_kv_heads) in (4, 8) and os.environ.get("HDS_GQA_PACKED", "1") != "0"
+
+
 def pick_group_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
     """KV splits of the grouped-query kernel (8 warps and one CTA per SM up to 148 CTAs, else 4 warps and two). Times at head_dim 128:
 
@@ -643,10 +651,10 @@ def pick_group_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
     return want
 
 
-def pick_small_splits(n_items: int, n_q_heads: int, n_kv_heads: int, max_kv_len: int) -> int:
-    """KV splits of a batch's small items, by the kernel that takes them: the one for query heads that share their keys (it reads a key
-    once for the group) or the one for heads of their own."""
-    return (pick_group_splits if n_q_heads > n_kv_heads else pick_decode_splits)(n_items, n_kv_heads, max_kv_len)
+def pick_small_splits(n_items: int, n_q_heads: int, n_kv_heads: int, head_dim: int, max_kv_len: int) -> int:
+    """KV splits of a batch's small items, by the kernel that takes them."""
+    pick = pick_group_splits if use_grouped_decode(n_q_heads, n_kv_heads, head_dim) else pick_decode_splits
+    return pick(n_items, n_kv_heads, max_kv_len)
 
 
 def pick_prefill_splits(n_items: int, n_q_heads: int, max_kv_len: int) -> int:

@@ -20,7 +20,8 @@
 // Measured on B200 (head_dim 128, bf16; before: 128-row tcgen05 tiles of the packed kernel):
 //   8 heads of 8 : 64 x 250 keys 34.4 -> 19.7 us, 8 x 4096: 42.8 -> 27.3, 1 x 16384: 30.4 -> 17.6
 //   4 heads of 4 : 8 x 600 keys 12.9 -> 8.3 us, 4 x 1024: 11.8 -> 7.5
-// Heads of their own keys and values (group size 1) stay with attention_splitkv.cu, whose weights are fp32 throughout.
+// Dispatched for groups of 4 and 8 heads at 128 dims, whose kernel before had 16-bit weights. All others stay with attention_splitkv.cu,
+// whose weights are fp32 throughout.
 //
 // Stands in for the external paged flash kernel the reference links
 // (deepspeed/inference/v2/kernels/ragged_ops/blocked_flash/blocked_flash.cpp:21-101, flash.h:74).

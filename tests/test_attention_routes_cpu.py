@@ -76,3 +76,22 @@ def test_no_scratch_no_split(n_q, n_kv, seqs, seen):
     assert [c.splits for c in launches(b, n_q, n_kv)] == [1]
     if seqs == 2:
         assert launches(b, n_q, n_kv, ws_small=torch.zeros(1), ws_large=torch.zeros(1))[0].splits > 1
+
+
+@pytest.mark.parametrize("n_q,n_kv,d,grouped", [(32, 8, 128, True), (64, 8, 128, True), (8, 1, 128, True), (4, 4, 128, False), (8, 4, 128, False),
+                                                (6, 2, 128, False), (10, 2, 128, False), (12, 2, 128, False), (14, 2, 128, False),
+                                                (32, 8, 64, False), (16, 2, 64, False)])
+def test_grouped_kernel_only_in_place_of_16_bit_weights(n_q, n_kv, d, grouped, monkeypatch):
+    """The kernel with weights in two 16-bit parts takes the groups whose weights were 16 bits before it: 4 and 8 at 128 dims. All others,
+    and all with HDS_GQA_PACKED=0, keep the kernel with fp32 weights, and its splits."""
+    from hcache_deepspeed_b200.ops import backend
+    ws = dict(ws_small=torch.zeros(1), ws_large=torch.zeros(1))
+    for seqs, seen in ((1, 100), (3, 3000), (60, 600)):
+        b = batch_of([(seen, 1)] * seqs, n_q // n_kv)
+        for env in ("1", "0"):
+            monkeypatch.setenv("HDS_GQA_PACKED", env)
+            want = grouped and env == "1"
+            c, = launches(b, n_q, n_kv, d, **ws)
+            pick = backend.pick_group_splits if want else backend.pick_decode_splits
+            assert c.name == "paged_attention_splitkv" and c.grouped == want and c.splits == pick(seqs, n_kv, seen + 1)
+            assert c.splits == backend.pick_small_splits(seqs, n_q, n_kv, d, seen + 1)
