@@ -12,7 +12,9 @@
 //     busier than the memory: 4.6 and 4.0 TB/s at 32 sequences x 32 heads x 1000 keys, where this has 6.1.)
 //   * The tensor cores do the arithmetic at any group size: 8 of the MMA's 16 rows are query rows. The other 8 take what
 //     rounding the weights to 16 bits leaves over, itself in 16 bits, so P V keeps the weights to 2^-16 and better in the same
-//     instruction. Scores, maxima, sums and outputs are fp32.
+//     instruction. fp16 would lose that, and at last the weight itself, below 2^-9, where its steps no longer shrink with the value:
+//     sigmoid weights are that small. There the weights go in times 2^14 (they are 1 at most), and the outputs come back by it: to
+//     2^-22 from 2^-17 on, no step above 2^-39. Scores, maxima, sums and outputs are fp32.
 //   * KV range is split over gridDim.z CTAs; partial (O, m, l) go to a scratch buffer and the last CTA to finish (atomic ticket)
 //     merges them: one launch, no separate combine kernel.
 //
@@ -102,6 +104,7 @@ paged_attn_group_kernel(const __grid_constant__ CUtensorMap tmap_kv, const Group
     constexpr int VC = D / 64;        // 16-byte pieces of a V row per lane
     constexpr int LD = D + 4;
     constexpr int ST = group_stages(D);
+    constexpr float kUp = kBf16 ? 1.0f : 16384.0f;      // what a weight is multiplied by before it becomes 16 bits
     static_assert(kGroupRows * LD * 4 <= ST * group_slot_bytes(D), "a warp's outputs fit its ring");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -253,6 +256,8 @@ paged_attn_group_kernel(const __grid_constant__ CUtensorMap tmap_kv, const Group
             }
         }
         // ---- O += P V: rounded weights in rows 0..7, what the rounding left in rows 8..15 ----
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] *= kUp;
         const uint32_t h0 = pack2<kBf16>(p[0], p[1]), h1 = pack2<kBf16>(p[2], p[3]);
         const uint32_t r0 = pack2<kBf16>(p[0] - unpack_lo<kBf16>(h0), p[1] - unpack_hi<kBf16>(h0));
         const uint32_t r1 = pack2<kBf16>(p[2] - unpack_lo<kBf16>(h1), p[3] - unpack_hi<kBf16>(h1));
@@ -300,8 +305,9 @@ paged_attn_group_kernel(const __grid_constant__ CUtensorMap tmap_kv, const Group
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 float4* d = reinterpret_cast<float4*>(mg_o(warp, g) + c * 64 + (2 * t + e) * 8);
-                d[0] = make_float4(acc[c][0][e] + acc[c][0][e + 2], acc[c][1][e] + acc[c][1][e + 2], acc[c][2][e] + acc[c][2][e + 2], acc[c][3][e] + acc[c][3][e + 2]);
-                d[1] = make_float4(acc[c][4][e] + acc[c][4][e + 2], acc[c][5][e] + acc[c][5][e + 2], acc[c][6][e] + acc[c][6][e + 2], acc[c][7][e] + acc[c][7][e + 2]);
+                auto sum = [&](int j) { return (acc[c][j][e] + acc[c][j][e + 2]) * (1.0f / kUp); };
+                d[0] = make_float4(sum(0), sum(1), sum(2), sum(3));
+                d[1] = make_float4(sum(4), sum(5), sum(6), sum(7));
             }
     }
     __syncthreads();

@@ -416,6 +416,31 @@ def test_attention_group_options(opts, n_q_heads, n_kv, d, bs, n_splits):
     torch.testing.assert_close(got.float(), want.float(), rtol=2.0**-7, atol=1e-3)     # each rounds its own outputs to bf16
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("bias", [-9.0, -12.0, -14.0])
+@pytest.mark.parametrize("n_q_heads,n_kv,d,n_splits", [(8, 2, 128, 1), (8, 1, 128, 5), (6, 2, 64, 1)])
+def test_attention_group_small_weights(dtype, bias, n_q_heads, n_kv, d, n_splits):
+    """Sigmoid weights down to 1e-7 keep their precision in the grouped kernel: large values times small weights against 64 bits. Besides
+    the output's own rounding, a weight is off by 2^-16 (bf16, two parts of 8 bits) or 2^-21 (fp16), and by what the fp32 score under
+    it is off (1e-5)."""
+    specs = [(0, 1), (15, 1), (333, 1), (900, 1)]
+    q, cache, tables, items = build_paged_problem(specs, n_q_heads, n_kv, d, 64, dtype, seed=10)
+    cache[:, 1] *= 256.0
+    items_t, G = torch.tensor(items, dtype=torch.int32, device="cuda"), n_q_heads // n_kv
+    vec = torch.linspace(bias - 1.0, bias + 1.0, n_q_heads, device="cuda")
+    ws = torch.zeros(max(K().splitkv_workspace_bytes(len(items), n_q_heads, n_kv, d, n_splits, G), 16), dtype=torch.uint8, device="cuda")
+    out = torch.zeros_like(q)
+    K().paged_attention_splitkv(q, out, cache, tables, items_t, len(items), G, n_q_heads, n_kv, d, 64, n_splits, 1 / math.sqrt(d), ws, sigmoid_bias=vec,
+                                grouped=True)
+    eps, per_weight = (2.0**-8, 2.0**-16) if dtype == torch.bfloat16 else (2.0**-11, 2.0**-21)
+    for (seq, row, n, pos0), t in zip(items, tables.tolist()):
+        pages = torch.cat([cache[b] for b in t[:(pos0 + n + 63) // 64]], 2).double().repeat_interleave(G, 1)
+        k, v = pages[0, :, :pos0 + 1], pages[1, :, :pos0 + 1]
+        p = torch.sigmoid((q[row].double()[:, None] * k).sum(-1) / math.sqrt(d) + vec.double()[:, None])[..., None]
+        want, size = (p * v).sum(1), (p * v.abs()).sum(1)
+        assert ((out[row].double() - want).abs() <= eps * want.abs() + (per_weight + 1e-5) * size + 2.0**-25).all()
+
+
 @pytest.mark.parametrize("n_q_heads,n_kv,d", [(8, 2, 128), (6, 2, 128), (4, 2, 64)])
 def test_attention_of_a_batch_for_smaller_groups(n_q_heads, n_kv, d):
     """Items of up to 8 tokens, as a batch built for heads of their own has them, under grouped attention: every row is computed."""
@@ -427,7 +452,7 @@ def test_attention_of_a_batch_for_smaller_groups(n_q_heads, n_kv, d):
                                   block_tables=lambda: tables, items_small=lambda: items_t)
     out = torch.full_like(q, float("nan"))
     CudaOps().attention(q.view(q.shape[0], -1), out.view(q.shape[0], -1), cache, batch, n_q_heads, n_kv, d, 1 / math.sqrt(d))
-    want = ref.paged_attention(q, cache, tables, items, n_q_heads, n_kv, 1 / math.sqrt(d))
+    want = ref.paged_attention(q, cache, tables, items_t.cpu(), n_q_heads, n_kv, 1 / math.sqrt(d))
     torch.testing.assert_close(out.float(), want.float(), **tol(torch.bfloat16))
 
 
