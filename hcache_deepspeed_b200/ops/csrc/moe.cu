@@ -254,13 +254,15 @@ __global__ void moe_gather_kernel(const void* __restrict__ y, int64_t ldy, const
 
 // The gather with a shared expert: out[t] += sum_j score[t, j] * y[row(t, j)] + sigmoid(x[t] . w_gate) * ys[t]. The gate's product
 // is H values per token, which the block of the token reads in passing; as operations of their own (widening copies, a product, a
-// sigmoid, a scaling, a sum) the gate and the sum took 26 us a layer at 16 tokens of width 4096, with the gather; this takes 6.
+// sigmoid, a scaling, a sum) the gate and the sum took 26 us a layer at 16 tokens of width 4096, with the gather; this takes 6. The gate's
+// weights may lie on any boundary of theirs (`wide`: on one of 16 bytes), as a slice of a flat parameter buffer does.
 template <bool kBf16>
 __global__ void __launch_bounds__(256)
 moe_gather_shared_kernel(const void* __restrict__ y, int64_t ldy, const int32_t* __restrict__ mapped_slots,
                          const float* __restrict__ scores, const void* __restrict__ x, int64_t ldx, const void* __restrict__ w_gate,
                          const void* __restrict__ ys, int64_t ldys, float* __restrict__ out, int64_t ldo, int H, int k) {
     __shared__ float red[8];
+    const bool wide = (reinterpret_cast<uintptr_t>(w_gate) & 15) == 0;
     const int64_t t = blockIdx.x;
     auto load8 = [](const void* p, int64_t idx, float (&v)[8]) {
         const uint4 q = *reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(p) + idx * 2);
@@ -272,7 +274,12 @@ moe_gather_shared_kernel(const void* __restrict__ y, int64_t ldy, const int32_t*
     for (int c = threadIdx.x * 8; c < H; c += 256 * 8) {
         float a[8], b[8];
         load8(x, t * ldx + c, a);
-        load8(w_gate, c, b);
+        if (wide) {
+            load8(w_gate, c, b);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) b[i] = load_scalar<kBf16>(w_gate, c + i);
+        }
 #pragma unroll
         for (int i = 0; i < 8; ++i) dot = fmaf(a[i], b[i], dot);
     }
@@ -371,6 +378,8 @@ extern "C" int hds_moe_gather_shared(const void* y, int64_t ldy, const int32_t* 
                                      int dtype, void* stream) {
     HDS_REQUIRE(H % 8 == 0 && ldy % 8 == 0 && ldx % 8 == 0 && ldys % 8 == 0 && ldo % 4 == 0, "hds_moe_gather_shared: H / strides must be vector aligned");
     HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_moe_gather_shared: dtype must be 0 (bf16) or 1 (fp16)");
+    HDS_REQUIRE(((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(ys) | reinterpret_cast<uintptr_t>(out)) & 15) == 0,
+                "hds_moe_gather_shared: rows on 16-byte boundaries");
     if (T == 0) return HDS_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (dtype == 0)

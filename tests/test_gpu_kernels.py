@@ -806,6 +806,22 @@ def test_gemm_2sm(dtype, M, N, K_, bn, mode):
     gated = mode == "gated"
     out = K().gemm_2sm(a, w, bias=b, act=3 if gated else 2, gated=gated, bn=bn)
     want = ref.gemm(a, w, bias=b, act=3 if gated else 2, gated=gated, out_dtype=torch.float32)
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_moe_gather_shared_boundaries(dtype):
+    """The gate's weights on any boundary, as a slice of a flat buffer: the same bits; rows that are not on 16 bytes are refused."""
+    T, k, H = 5, 2, 264
+    x, y, ys, flat = rand(T, H, dtype=dtype), rand(64, H, dtype=dtype), rand(T, H, dtype=dtype), rand(H + 8, dtype=dtype)
+    slots, scores = torch.randint(0, 64, (T, k), device="cuda", dtype=torch.int32), torch.rand(T, k, device="cuda")
+    for off in (1, 3, 4):
+        outs = []
+        for gate in (flat[off:off + H], flat[off:off + H].clone()):
+            outs.append(torch.zeros(T, H, device="cuda"))
+            K().moe_gather_shared(y, slots, scores, x, gate.view(1, H), ys, outs[-1])
+        assert torch.equal(*outs)
+    with pytest.raises(RuntimeError, match="16-byte"):
+        K().moe_gather_shared(y, slots, scores, rand(T * H + 1, dtype=dtype)[1:].view(T, H), flat[:H].view(1, H), ys, outs[0])
+
+
     torch.testing.assert_close(out.float(), want, **tol(dtype))
 
 
