@@ -37,7 +37,8 @@ __host__ __device__ constexpr size_t skinny_smem_bytes(int nt, bool grouped = fa
 
 // K splits of a decode GEMM of n_tiles feature tiles. Measured (profiles/kernel_bench_decode_gemm.jsonl): fill the resident slots once;
 // past one full wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4
-// splits). At most 8, the size of a portable cluster. A cluster needs its slots in one GPC, so that some stay empty: where the splits
+// splits). At most 8, the size of a portable cluster; a count that the caller gives is held to that where the splits meet in one (`clusters`),
+// and to the K blocks where they add up in memory. A cluster needs its slots in one GPC, so that some stay empty: where the splits
 // meet in one, they fill no more than 87 % (96 tiles x 3 of 296 slots: 27.7 us at 17 tokens of 12288 x 4096, 20.4 us in 2).
 inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms, bool clusters) {
     int splits = want;
@@ -59,7 +60,7 @@ inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms, b
         }
         if (splits > kb_total / 4) splits = kb_total / 4;
     }
-    if (splits > 8) splits = 8;
+    if (splits > 8 && (clusters || want <= 0)) splits = 8;
     if (splits > kb_total) splits = kb_total;
     return splits < 1 ? 1 : splits;
 }

@@ -326,6 +326,17 @@ def test_gemm_cluster_splits(dtype, M, N, K_, splits, gated):
     torch.testing.assert_close(out.float(), want, **tol(dtype))
 
 
+@pytest.mark.parametrize("splits,kept", [(16, 0.0), (8, 16.0), (1, 16.0)])
+def test_gemm_accum_explicit_splits(splits, kept):
+    """As many K splits of an accumulating product as the caller asks for, past the 8 that a cluster holds: sixteen ones that come one by
+    one are lost beside 2^24, in pairs or as one sum they are not."""
+    a, w = torch.zeros(1, 1024, dtype=torch.bfloat16, device="cuda"), torch.ones(128, 1024, dtype=torch.bfloat16, device="cuda")
+    a[0, ::64] = 1.0
+    acc = torch.full((1, 128), 2.0**24, device="cuda")
+    K().gemm_accum(a, w, acc, bn=-1, splits=splits)
+    assert bool((acc - 2.0**24 == kept).all())
+
+
 # ------------------------------------------------------------------------------------------------
 # paged attention
 # ------------------------------------------------------------------------------------------------
