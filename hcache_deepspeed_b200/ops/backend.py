@@ -628,17 +628,18 @@ def use_grouped_decode(n_q_heads: int, n_kv_heads: int, head_dim: int) -> bool:
 def pick_group_splits(n_items: int, n_kv_heads: int, max_kv_len: int) -> int:
     """KV splits of the grouped-query kernel (8 warps and one CTA per SM up to 148 CTAs, else 4 warps and two). Times at head_dim 128:
 
-    * up to half as many (item, KV head) pairs as SMs: one wave of CTAs, at least 128 keys (a strip per warp) each. 8 pairs of 16384
-      keys: 132.6 us unsplit, 17.6 in 16; 64 of 4096: 37.6 unsplit, 27.3 in 2; 16 of 1024: 12.1 unsplit, 7.5 in 8. Under 512 keys
-      merging costs what it gains (16 of 300: 6.5 us unsplit, 7.0 in 3).
+    * up to half as many (item, KV head) pairs as SMs: one wave of CTAs. 8 pairs of 16384 keys: 132.6 us unsplit, 17.6 in 16; 64 of
+      4096: 37.6 unsplit, 27.3 in 2; 16 of 1024: 12.1 unsplit, 7.5 in 8. Under 512 keys merging costs what it gains (16 of 300: 6.5 us
+      unsplit, 7.0 in 3). A growing context asks for another CUDA graph with every other split count, so that there are two: 8, and 16
+      from 2048 keys on (8 pairs of 520 / 1000 / 1500 / 1900 keys: 6.7 / 7.0 / 7.9 / 8.2 us in 8, 7.3 / 7.7 / 8.9 / 9.9 in 4,
+      7.3 / 7.6 / 8.6 / 8.8 in one per 128 keys, 7.3 / 7.6 / 8.0 / 8.2 in 16).
     * up to the 296 slots: no split (96 of 700 keys: 10.5 us, 12.6 in 2; 256 of 800: 21.1 us, 26.7 in 2).
     * beyond: a last wave that is nearly empty costs up to half the rate (320 of 2000 keys: 76.0 us unsplit, 65.1 in 4), so the fewest
       splits whose waves are 85 % full, of at least 512 keys (320 of 400: 20.8 us unsplit, 28.5 in 4)."""
     ctas = max(1, n_items * n_kv_heads)
     slots = 2 * N_SM
     if ctas <= N_SM:
-        cap = max_kv_len // 128 if max_kv_len >= 512 else 1
-        return int(max(1, min(N_SM // ctas, cap, MAX_DECODE_SPLITS)))
+        return min(N_SM // ctas, 16 if max_kv_len >= 2048 else 8 if max_kv_len >= 512 else 1)
     if ctas <= slots:
         return 1
     want, best = 1, 0.0

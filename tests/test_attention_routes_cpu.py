@@ -95,3 +95,11 @@ def test_grouped_kernel_only_in_place_of_16_bit_weights(n_q, n_kv, d, grouped, m
             pick = backend.pick_group_splits if want else backend.pick_decode_splits
             assert c.name == "paged_attention_splitkv" and c.grouped == want and c.splits == pick(seqs, n_kv, seen + 1)
             assert c.splits == backend.pick_small_splits(seqs, n_q, n_kv, d, seen + 1)
+
+
+@pytest.mark.parametrize("n_items,n_kv", [(1, 8), (4, 4), (1, 2), (9, 8)])
+def test_split_counts_of_a_growing_context(n_items, n_kv):
+    """Every split count is a CUDA graph of its own: a context that grows from nothing to 16384 keys passes three of them at most."""
+    from hcache_deepspeed_b200.ops.backend import pick_group_splits
+    counts = [pick_group_splits(n_items, n_kv, n) for n in range(1, 16385)]
+    assert len(set(counts)) <= 3 and counts == sorted(counts) and max(counts) * n_items * n_kv <= 148
