@@ -241,15 +241,15 @@ def norm(x: torch.Tensor, gamma: torch.Tensor, out: torch.Tensor, *, beta: Optio
     :func:`quantize_fp8_rows` would make of ``out``."""
     cols = x.shape[-1]
     n = rows if rows is not None else (row_idx.numel() if row_idx is not None else x.numel() // cols)
-    lib = native.cuda_lib()
-    if fp8 is not None:
+    lib, dt, stream = native.cuda_lib(), _dt(x), _stream()
+    if fp8 is not None:       # (last: what is armed has to meet its norm)
         q, scales = fp8
         assert q.dtype == torch.uint8 and scales.dtype == torch.float32 and q.shape == (n, cols) and scales.numel() >= n and scales.is_contiguous()
         native.check(lib.hds_norm_next_fp8(_p(q), q.stride(0), _p(scales)), "hds_norm_next_fp8")
     rc = lib.hds_norm(_p(x), x.stride(-2) if x.dim() > 1 else cols, _p(delta),
                       1 if (delta is not None and delta.dtype == torch.float32) else 0, 1 if zero_delta else 0,
                       _p(res_out), _p(out), out.stride(-2) if out.dim() > 1 else cols, _p(gamma), _p(beta), _p(row_idx),
-                      n, cols, eps, 1 if layer_norm else 0, 1 if post_norm else 0, _dt(x), _stream())
+                      n, cols, eps, 1 if layer_norm else 0, 1 if post_norm else 0, dt, stream)
     native.check(rc, "hds_norm")
     _count()
     return out
