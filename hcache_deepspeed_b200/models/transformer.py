@@ -461,7 +461,8 @@ class RaggedTransformer:
             k.moe_gemm(hs, st["w_down"], st["pad_off"], E, ys, choices=T * kk)
             if lw.shared_expert is not None:
                 se = lw.shared_expert
-                act = self.act_buf[:T, :se.w_up.shape[0] // mult]
+                n_act = se.w_up.shape[0] // mult     # (rows of its own width: the buffer's may be no multiple of 8)
+                act = self.act_buf.view(-1)[:T * n_act].view(T, n_act)
                 self.ops.gemm(x, se.w_up, act, act=self.act, gated=s.gated_mlp, workspace=self.ws_gemm)
                 shared = self.ops.gemm(act, se.w_down, self.delta16[:T, :s.hidden], workspace=self.ws_gemm)
                 k.moe_gather_shared(ys, st["mapped_slots"][:T], st["scores"][:T], x, lw.w_shared_gate, shared, d32)

@@ -35,6 +35,39 @@ def test_gpu_matches_cpu_oracle(arch):
         torch.testing.assert_close(lg.float().cpu(), lc, rtol=5e-2, atol=5e-2)
 
 
+def _shared_expert_moe(dense=140, hidden=256):
+    """A small Qwen2-MoE (shared expert behind a gate) whose dense, expert and shared sizes differ; experts are alike but for a tenth, so
+    that a near-tie of the router does no harm."""
+    import transformers as tf
+    torch.manual_seed(3)
+    m = tf.Qwen2MoeForCausalLM(tf.Qwen2MoeConfig(
+        intermediate_size=dense, moe_intermediate_size=64, shared_expert_intermediate_size=136, num_experts=6, num_experts_per_tok=2,
+        num_key_value_heads=2, decoder_sparse_step=1, norm_topk_prob=True, vocab_size=300, hidden_size=hidden, num_hidden_layers=2,
+        num_attention_heads=4, max_position_embeddings=1024)).eval()
+    with torch.no_grad():
+        for name, p in m.named_parameters():
+            if p.dim() == 3:
+                p.copy_(p[:1] + 0.1 * (p - p[:1]))
+            elif p.dim() == 2:
+                p.mul_(2.0)
+    return m
+
+
+def test_shared_expert_matches_cpu_oracle():
+    """A mixture of experts with a shared expert, on both sides of 64 choices and of 64 and 128 tokens. The dense size, which no layer of
+    the model uses, is the widest and no multiple of 8: nothing may hang on it."""
+    from hcache_deepspeed_b200.inference.v2.engine_factory import build_engine_from_module
+    m = _shared_expert_moe().to(torch.bfloat16)
+    gpu = build_engine_from_module(m, _cfg(), dtype=torch.bfloat16, device=torch.device("cuda"))
+    cpu = build_engine_from_module(m.float(), _cfg(mem=64 * 1024 * 1024), dtype=torch.float32, device=torch.device("cpu"))
+    g = torch.Generator().manual_seed(1)
+    for uid, n in enumerate((1, 31, 33, 64, 65, 128, 200)):
+        ids = torch.randint(0, 300, (n, ), generator=g)
+        for step in (ids, ids[:1]):
+            lg, lc = gpu.put([uid], [step])[0], cpu.put([uid], [step])[0]
+            torch.testing.assert_close(lg.float().cpu(), lc, rtol=5e-2, atol=5e-2)
+
+
 def test_restore_equals_live_kv_llama7b_shapes():
     from hcache_deepspeed_b200.inference.v2 import build_engine_from_arch
     from hcache_deepspeed_b200.models.arch import named_arch
