@@ -450,7 +450,9 @@ class RaggedTransformer:
             k = self.ops.k
             E, kk = len(lw.experts), s.top_k
             st = self._moe_state(lw, E, kk)
-            logits = k.gemm(x, lw.w_router, out=st["logits"][:T], workspace=self.ws_gemm)
+            # (no scratch: above 64 tokens its split sums meet in the order of their arrival, and a near-tie of experts would not be the
+            # same from run to run)
+            logits = k.gemm(x, lw.w_router, out=st["logits"][:T])
             k.moe_topk_gating(logits, kk, s.norm_topk_prob, st["scores"][:T], st["expert_ids"][:T], st["offsets"][:T],
                               st["counts"])
             rows = k.moe_padded_rows(T, E, kk)

@@ -68,6 +68,24 @@ def test_shared_expert_matches_cpu_oracle():
             torch.testing.assert_close(lg.float().cpu(), lc, rtol=5e-2, atol=5e-2)
 
 
+def test_router_sums_in_a_fixed_order():
+    """The router's logits decide between experts, so that an input gives the same ones every time: each is one sum over the width, in
+    order, at 65 to 128 tokens as at all others. The sums here depend on the order: what lies between the two large terms is lost
+    unless it is summed apart from them."""
+    from hcache_deepspeed_b200.inference.v2.engine_factory import build_engine_from_module
+    from hcache_deepspeed_b200.ops import kernels as K
+    model = build_engine_from_module(_shared_expert_moe(hidden=2048).to(torch.bfloat16), _cfg(), dtype=torch.bfloat16, device=torch.device("cuda")).model()
+    lw = model.w.layers[0]
+    lw.w_router = (2.0**torch.arange(6, device="cuda")).to(torch.bfloat16)[:, None].repeat(1, 2048)
+    for T in (100, 128):
+        x = torch.full((T, 2048), 2.0**-8, dtype=torch.bfloat16, device="cuda")
+        x[:, 0], x[:, -1] = 2.0**20, -2.0**20
+        want = K.gemm(x, lw.w_router)
+        for _ in range(3):
+            model._moe(x, lw, T)
+            assert torch.equal(model._moe_bufs["logits"][:T], want)
+
+
 def test_restore_equals_live_kv_llama7b_shapes():
     from hcache_deepspeed_b200.inference.v2 import build_engine_from_arch
     from hcache_deepspeed_b200.models.arch import named_arch
