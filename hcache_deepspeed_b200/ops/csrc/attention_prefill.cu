@@ -529,7 +529,7 @@ static int launch_prefill64(const CUtensorMap& tq, const CUtensorMap& tkv, const
     return HDS_OK;
 }
 
-// Measured (tools/prefill64_probe.sh, 4224 causal tokens x 32 heads x d128): 292 us (515 TFLOP/s) against 302 us (498) for the
+// Measured (4224 causal tokens x 32 heads x d128): 292 us (515 TFLOP/s) against 302 us (498) for the
 // 128-key kernel, and 53.7 ms against 51.8 ms for a whole fresh 4160-token Llama-2-7B prefill: two co-resident CTAs do not buy
 // the overlap that was hoped for, so the 128-key kernel stays the default and this shape is opt-in (HDS_PREFILL_TILE=64).
 static bool prefill64_enabled() {
@@ -559,10 +559,9 @@ static int launch_pair(const CUtensorMap& tq, const CUtensorMap& tkv, const Pref
 }
 
 // Two heads of a group per CTA: head_dim 128, an even group, no ALiBi, no KV split, and at least as many pairs as SMs (at 12 items of
-// 128 tokens x 32 heads, 192 pairs, 28.2 -> 26.9 us; with fewer, one head per CTA keeps more SMs busy).
+// 128 tokens x 32 heads, 192 pairs, 28.2 -> 26.9 us; with fewer, one head per CTA keeps more SMs busy). Not where 64-key tiles are asked for.
 static bool use_pair(const PrefillArgs& a, int head_dim, int n_items) {
-    static const int on = getenv("HDS_ATTN_PAIR") ? atoi(getenv("HDS_ATTN_PAIR")) : 1;
-    return on && head_dim == 128 && (a.n_q_heads / a.n_kv_heads) % 2 == 0 && a.alibi == nullptr && a.n_splits == 1 &&
+    return !prefill64_enabled() && head_dim == 128 && (a.n_q_heads / a.n_kv_heads) % 2 == 0 && a.alibi == nullptr && a.n_splits == 1 &&
            static_cast<int64_t>(n_items) * (a.n_q_heads / 2) >= sm_count();
 }
 

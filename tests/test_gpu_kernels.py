@@ -383,8 +383,8 @@ def test_attention_splitkv_decode(dtype, n_q_heads, n_kv, d, bs, n_splits):
                                                                (2, 2, 64, 32, 9, False), (10, 2, 64, 128, 1, True), (21, 3, 128, 64, 2, True)])
 def test_attention_group_strips(dtype, n_q_heads, n_kv, d, bs, n_splits, many):
     """Ends of the 16-key strips, fewer strips than warps or splits, every row count of a group, CTAs of eight warps and (``many``: more
-    than 148 of them) of four. Rows behind a sequence's last key are not numbers; outputs keep fp32 weights, so only their own
-    rounding to 16 bits (and the products' order) separates them from 64 bits."""
+    than 148 of them) of four. Rows behind a sequence's last key are not numbers. Weights in two 16-bit parts are off by 2^-16 of
+    themselves at most, so that the outputs' own rounding to 16 bits is what separates them from 64 bits."""
     specs = [(c, 1) for c in (0, 14, 15, 16, 30, 31, 47, 63, 64, 127, 500)] * (16 if many else 1) + [(40, 8 // (n_q_heads // n_kv))]
     q, cache, tables, items = build_paged_problem(specs, n_q_heads, n_kv, d, bs, dtype, seed=5)
     for (seq, _, n, pos0), t in zip(items, tables.tolist()):
@@ -659,6 +659,37 @@ def test_attention_prefill_64_key_tiles_subprocess():
                           "--timeout", "120", "-p", "no:cacheprovider"], env=env, capture_output=True, text=True, timeout=300)
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-1000:]
     assert " passed" in res.stdout
+
+
+_SWITCH_PROBES = {
+    "attention": """
+q, cache, tables, items = t.build_paged_problem([(0, 128)] * 20, 16, 4, 128, 64)
+it = torch.tensor(items, dtype=torch.int32, device="cuda")
+call = lambda: t.K().paged_attention_prefill(q, torch.empty_like(q), cache, tables, it, len(items), 16, 4, 128, 64, 0.09)
+""",
+}
+
+
+@pytest.mark.parametrize("probe,var,value,kernel", [("attention", "HDS_PREFILL_TILE", "64", "paged_attn_prefill64_kernel"),
+                                                    ("attention", "HDS_PREFILL_TILE", "128", "paged_attn_pair_kernel")])
+def test_switches_read_once_per_process(probe, var, value, kernel):
+    """Environment switches that choose a kernel: the kernel that a child process with the variable set really runs."""
+    import os
+    import subprocess
+    import sys
+    code = f"""
+import sys, torch
+sys.path.insert(0, {os.path.dirname(os.path.abspath(__file__))!r}); sys.path.insert(0, {os.path.dirname(os.path.dirname(os.path.abspath(__file__)))!r})
+import test_gpu_kernels as t
+{_SWITCH_PROBES[probe]}
+call(); torch.cuda.synchronize()
+with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+    call(); torch.cuda.synchronize()
+print([e.key for e in p.key_averages()])
+"""
+    res = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **{var: value}), capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+    assert kernel in res.stdout
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
