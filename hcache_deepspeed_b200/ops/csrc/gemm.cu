@@ -375,6 +375,7 @@ extern "C" int hds_moe_gemm_few(const void* A, int64_t lda, const void* W_stacke
     HDS_REQUIRE(n_experts >= 1 && pad_off != nullptr && max_rows % kGemmBM == 0,
                 "hds_moe_gemm_few: needs expert offsets and a row capacity that is a multiple of 128");
     HDS_REQUIRE(max_per_expert >= 1 && max_per_expert <= 64 && max_experts >= 1, "hds_moe_gemm_few: 1..64 rows per expert");
+    if (!skinny_enabled()) return hds_moe_gemm(A, lda, W_stacked, ldw, pad_off, n_experts, max_rows, N, K, dtype, epilogue, act, out, ldo, stream);
     HDS_REQUIRE(N > 0 && K > 0 && K % 8 == 0 && lda % 8 == 0 && ldw % 8 == 0, "hds_moe_gemm_few: K, lda, ldw must be multiples of 8 elements");
     HDS_REQUIRE(epilogue != EPI_GATED || (N % 2 == 0), "hds_moe_gemm_few: gated epilogue needs an even N");
     const int nt = skinny_nt(max_per_expert);

@@ -667,11 +667,16 @@ q, cache, tables, items = t.build_paged_problem([(0, 128)] * 20, 16, 4, 128, 64)
 it = torch.tensor(items, dtype=torch.int32, device="cuda")
 call = lambda: t.K().paged_attention_prefill(q, torch.empty_like(q), cache, tables, it, len(items), 16, 4, 128, 64, 0.09)
 """,
+    "experts": """
+x, w, pad = torch.zeros(256, 128, dtype=torch.bfloat16, device="cuda"), t.rand(256, 128), torch.tensor([0, 128, 256], dtype=torch.int32, device="cuda")
+call = lambda: t.K().moe_gemm(x, w, pad, 2, torch.empty(256, 128, dtype=torch.bfloat16, device="cuda"), choices=8)
+""",
 }
 
 
 @pytest.mark.parametrize("probe,var,value,kernel", [("attention", "HDS_PREFILL_TILE", "64", "paged_attn_prefill64_kernel"),
-                                                    ("attention", "HDS_PREFILL_TILE", "128", "paged_attn_pair_kernel")])
+                                                    ("attention", "HDS_PREFILL_TILE", "128", "paged_attn_pair_kernel"),
+                                                    ("experts", "HDS_GEMM_SKINNY", "0", "gemm_tn_kernel"), ("experts", "HDS_GEMM_SKINNY", "1", "gemm_skinny_kernel")])
 def test_switches_read_once_per_process(probe, var, value, kernel):
     """Environment switches that choose a kernel: the kernel that a child process with the variable set really runs."""
     import os
