@@ -1,6 +1,6 @@
 """Per-kernel timing on one B200: CUDA events, >=3 warm-ups, L2 flushed between timed iterations.
-Prints one JSON line per case and writes gpurun_out/kernel_bench.jsonl. Roofline fractions are
-against MEASURED_PEAKS.json (measured copy bandwidth / cuBLAS bf16), fallback 6650 GB/s, 1590 TFLOP/s.
+Prints one JSON line per case. Roofline fractions are
+against the peaks measured on the machine where they are known (measured copy bandwidth / cuBLAS bf16), fallback 6650 GB/s, 1590 TFLOP/s.
 """
 import json
 import math
@@ -238,7 +238,3 @@ if __name__ == "__main__":
              "attn_decode": bench_attention_decode, "tiled": bench_tiled, "attn_prefill": bench_attention_prefill, "norm": bench_norm, "gemm_fp8": bench_gemm_fp8}
     for w in which:
         table[w]()
-    os.makedirs("gpurun_out", exist_ok=True)
-    with open("gpurun_out/kernel_bench.jsonl", "a") as f:
-        for r in results:
-            f.write(json.dumps(r) + "\n")
