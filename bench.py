@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Headline benchmark: restored multi-turn sessions on the ragged engine (BASELINE.json config 2..5).
+"""Headline benchmark: restored multi-turn sessions on the ragged engine.
 
 One STEP = one serving round over B synthetic multi-turn sessions:
   for each session: restore_kv(4K-token context from the pinned host hidden-state cache)  -> H2D + K/V projection
@@ -62,7 +62,7 @@ def parse():
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons sampled during the timed region (B200_PROFILING.md recipe)."""
+    """nvidia-smi clocks / throttle reasons sampled during the timed region."""
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,clocks_event_reasons.hw_slowdown,"
          "clocks_event_reasons.hw_thermal_slowdown,clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
 

@@ -1,6 +1,6 @@
 """hcache_deepspeed_b200 — a B200-native (sm_100a) LLM inference / serving framework with the capabilities of
 the HCache fork of DeepSpeed. Top-level API mirrors ``deepspeed/__init__.py`` (``init_inference`` :291,
-``init_distributed`` :43, ``add_config_arguments`` :268, ``initialize`` :69). See DESIGN.md."""
+``init_distributed`` :43, ``add_config_arguments`` :268, ``initialize`` :69)."""
 from __future__ import annotations
 
 import json

@@ -6,7 +6,7 @@ captures FX graphs, passes rewrite them at given training steps, and custom ops 
 traced or code-generated: the ZeRO-3 hooks record the module order of one profiled iteration, the passes compute a
 schedule on that order (which gathers to launch when, which parameters to keep resident, when optimizer states
 move), and the schedule is written back into the hook installer and the optimizer. Collectives stay NCCL calls on
-their own streams; launch-bound regions are CUDA-graphed elsewhere (see DESIGN.md)."""
+their own streams; launch-bound regions are CUDA-graphed elsewhere."""
 from __future__ import annotations
 
 import time

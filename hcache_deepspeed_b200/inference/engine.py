@@ -11,7 +11,7 @@ Counterpart of ``deepspeed/inference/engine.py:40-625``. Modes:
   as in the reference.
 
 New relative to the reference: sessions (``session_ids=``) and hidden-state save / restore on the v1 API
-(``hidden_states`` / ``restore_hidden_states``) — BASELINE.json config 1.
+(``hidden_states`` / ``restore_hidden_states``).
 """
 from __future__ import annotations
 

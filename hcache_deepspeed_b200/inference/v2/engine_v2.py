@@ -5,7 +5,7 @@ Public surface of the reference's ``InferenceEngineV2`` (``deepspeed/inference/v
 (lines 107-128), ``query``, ``can_schedule``, ``get_remaining_block_capacity``, ``flush``, ``serialize``,
 ``free_blocks``, ``n_kv_cache_groups``, ``model``.
 
-Defects of the fork that are NOT reproduced (SURVEY §2.1):
+Defects of the fork that are NOT reproduced:
 * ``put`` works for every model family, not only Llama-2 (the fork unpacks a 2-tuple that only the Llama
   model returns);
 * ``restore_kv`` skips ``None`` latents without dereferencing missing sequences, and compares with ``is None``

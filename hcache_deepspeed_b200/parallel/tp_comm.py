@@ -116,7 +116,7 @@ class FlagTPComm(TPComm):
         except Exception:
             pass
 
-    #: experiments only (tools/tp_decode_probe.py): drop every wait and signal — results are WRONG, timing shows what the
+    #: experiments only: drop every wait and signal — results are WRONG, timing shows what the
     #: flag exchanges cost
     debug_nosync = False
 

@@ -1,4 +1,4 @@
-"""``init_inference`` (v1 API) on CPU — BASELINE.json config 1: an OPT-shaped model, one rank, hidden states saved for a
+"""``init_inference`` (v1 API) on CPU: an OPT-shaped model, one rank, hidden states saved for a
 512-token context, KV rebuilt from them, logits compared with recompute. Also the config rules of
 ``deepspeed/__init__.py:341-362`` and ``inference/config.py`` (conflicts, deprecated aliases), generate(), beams."""
 import pytest
