@@ -337,10 +337,13 @@ extern "C" int hds_gemm_accum(const void* A, int64_t lda, const void* W, int64_t
     HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_gemm_accum: dtype must be 0 (bf16) or 1 (fp16)");
     HDS_REQUIRE(n_targets >= 1 && n_targets <= kMaxPeers, "hds_gemm_accum: 1..8 accumulation targets");
     HDS_REQUIRE(red_mode >= 0 && red_mode <= 2, "hds_gemm_accum: red_mode 0 (local) / 1 (p2p) / 2 (multicast)");
-    // (as the stores: 64 tokens, token-major against feature-major: 8192 x 28672 79.1 and 73.3 us, 8192 x 8192 25.5 and 23.4, 4096 x 4096
-    // 10.0 and 9.7, 2048 x 2048 6.0 and 5.7; but 1280 x 8192 8.2 and 9.9, and 9.0 and 8.4 at 32 tokens)
-    if (M <= 64 && ldw >= 0 && red_mode == 0 && n_targets == 1 &&
-        (bn == -1 || (bn == 0 && skinny_enabled() && (M <= 32 || N >= 2048))))
+    // As the stores, but for narrow outputs: a few feature tiles in 8 splits each are fewer CTAs than the token-major kernel's 64-wide tiles
+    // in more splits, which need not meet here. Token-major against feature-major, us: 32 tokens, 64 x 4096 3.3 and 4.6, 512 x 4096 4.4 and
+    // 4.8, 512 x 8192 5.5 and 7.0, 1024 x 4096 5.5 and 4.9, 1024 x 8192 7.7 and 7.8, 4096 x 4096 9.7 and 8.6. 64 tokens, 1536 x 4096 6.8
+    // token-major, 2048 x 4096 7.4 and 7.4, 2048 x 8192 10.2 and 11.0, 2752 x 8192 12.3 and 12.8, 4096 x 8192 16.0 and 15.5, 8192 x 28672
+    // 79.1 and 73.3.
+    const bool wide = M <= 16 || (M <= 32 ? N >= 1024 : N >= (K <= 4096 ? 2048 : 4096));
+    if (M <= 64 && ldw >= 0 && red_mode == 0 && n_targets == 1 && (bn == -1 || (bn == 0 && skinny_enabled() && wide)))
         return launch_skinny(EPI_RED_F32, dtype == 0, A, lda, W, ldw, M, N, K, 0, bias, nullptr, 0, accum_ptrs[0],
                              ld_accum, splits, static_cast<cudaStream_t>(stream));
     GemmArgs g;

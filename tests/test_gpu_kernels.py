@@ -337,6 +337,50 @@ def test_gemm_accum_explicit_splits(splits, kept):
     assert bool((acc - 2.0**24 == kept).all())
 
 
+def kernels_of(calls):
+    """The kernels that each of ``calls`` (expressions over this module as ``t``) launches, as a child process sees them."""
+    import json
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = f"""
+import json, sys, torch
+sys.path[:0] = [{here!r}, {os.path.dirname(here)!r}]
+import test_gpu_kernels as t
+out = []
+for c in json.loads({json.dumps(json.dumps(calls))}):
+    eval(c); torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        eval(c); torch.cuda.synchronize()
+    out.append(" ".join(e.key for e in p.key_averages()))
+print(json.dumps(out))
+"""
+    res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr[-2000:]
+    return json.loads(res.stdout.splitlines()[-1])
+
+
+ACCUM_RULE = [(16, 64, 4096, "gemm_skinny"), (17, 16, 2048, "gemm_tn"), (32, 1016, 4096, "gemm_tn"), (32, 1024, 8192, "gemm_skinny"), (33, 2048, 4096, "gemm_skinny"),
+              (33, 2040, 4096, "gemm_tn"), (64, 2048, 4104, "gemm_tn"), (64, 4096, 8192, "gemm_skinny")]
+
+
+@pytest.mark.parametrize("M,N,K_,_", ACCUM_RULE)
+def test_gemm_accum_around_the_rule(M, N, K_, _):
+    torch.manual_seed(M + N)
+    a, w, base = rand(M, K_), rand(N, K_, scale=K_ ** -0.5), torch.randn(M, N, device="cuda")
+    acc = base.clone()
+    K().gemm_accum(a, w, acc)
+    torch.testing.assert_close(acc, base + ref.gemm(a, w, out_dtype=torch.float32), rtol=1e-4, atol=2e-4)     # fp32 sums of up to 8192 products
+
+
+def test_gemm_accum_rule():
+    """On both sides of each line of the rule: the kernel that runs."""
+    ran = kernels_of([f"t.K().gemm_accum(t.rand({M}, {K_}), t.rand({N}, {K_}), torch.zeros({M}, {N}, device='cuda'))" for M, N, K_, _ in ACCUM_RULE])
+    for names, case in zip(ran, ACCUM_RULE):
+        assert case[3] in names, case
+
+
 # ------------------------------------------------------------------------------------------------
 # paged attention
 # ------------------------------------------------------------------------------------------------
