@@ -874,6 +874,16 @@ def test_norm_fp8(dtype, rows, cols, layer):
     assert torch.equal(s, want) and torch.equal(q, (wide.float() * inv[:, None]).to(torch.float8_e4m3fn).view(torch.uint8))
 
 
+@pytest.mark.parametrize("K_", [768, 2048, 4096, 8184, 8192, 16384])
+def test_quantize_fp8_many_rows(K_):
+    """More rows than SMs take other numbers of threads: a row's codes and scale are the same, bit for bit, as in a launch of a few."""
+    x = rand(300, K_) * torch.linspace(0.0, 3.0, 300, device="cuda")[:, None].bfloat16()
+    q, s = K().quantize_fp8_rows(x)
+    for r in range(0, 300, 100):
+        q1, s1 = K().quantize_fp8_rows(x[r:r + 100])
+        assert torch.equal(q[r:r + 100], q1) and torch.equal(s[r:r + 100], s1)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("T,k,H", [(1, 1, 8), (5, 2, 2056), (33, 4, 4096)])
 def test_moe_gather_shared(dtype, T, k, H):
