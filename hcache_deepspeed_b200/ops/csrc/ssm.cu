@@ -232,9 +232,16 @@ __global__ void __launch_bounds__(kScanWarps * 32) ssm_scan_kernel(const SsmArgs
 }
 
 // ---- one token per sequence --------------------------------------------------------------------------------------
-// Threads: a warp per 4 state rows, 16 warps at most.
+// Threads: a warp per 4 state rows, 16 warps at most, as long as the CTAs are few and a row's chain is what bounds. With more CTAs than
+// run at once, their number does: fewer warps each then. Heads of 64 x 128, us with 512 / 256 / 128 threads: 256 CTAs 6.8 / 9.4 / 11.2, 512
+// CTAs 12.1 / 10.7 / 15.0, 768 CTAs 16.7 / 16.4 / 16.5, 1024 CTAs 21.4 / 18.9 / 18.2, 8192 CTAs 130.7 / 114.2 / 105.5; before, with 128
+// threads that loaded after the convolution, 12.6, 14.5, 17.0, 19.2 and 127.1.
 constexpr int kStepRows = 4, kStepMaxThreads = 512;
-static int step_threads(int P) { return P >= 64 ? 512 : P >= 32 ? 256 : 128; }
+static int step_threads(int P, int64_t ctas) {
+    const int sms = sm_count(), rows = P >= 64 ? 512 : P >= 32 ? 256 : 128;
+    const int most = ctas <= 2 * sms ? 512 : ctas <= 6 * sms ? 256 : 128;
+    return rows < most ? rows : most;
+}
 
 // CTA = (sequence, head). The convolution of the head's x channels and its group's B and C is redone per head (a few taps);
 // VEC4: state rows are read and written as float4 (N a multiple of 4).
@@ -361,7 +368,7 @@ template <int DT>
 static int launch_step(const SsmArgs& a, cudaStream_t s) {
     const dim3 grid(a.n_seqs, a.heads);
     const size_t smem = static_cast<size_t>(2 * a.N + a.P) * 4;
-    const dim3 block(step_threads(a.P));
+    const dim3 block(step_threads(a.P, static_cast<int64_t>(a.n_seqs) * a.heads));
     if (a.N % 4 == 0) HDS_CHECK_CUDA(launch_kernel(ssm_step_kernel<DT, true>, grid, block, smem, s, a));
     else HDS_CHECK_CUDA(launch_kernel(ssm_step_kernel<DT, false>, grid, block, smem, s, a));
     return HDS_OK;

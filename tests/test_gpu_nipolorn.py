@@ -154,6 +154,29 @@ def test_state_space_against_reference(heads, P, N, groups, taps, dtype, method)
             torch.testing.assert_close(ring[s].cpu()[filled], ring_ref[s][filled])
 
 
+@pytest.mark.parametrize("heads,P,N,seqs", [(24, 64, 128, 13), (24, 64, 128, 38), (8, 100, 32, 38), (8, 32, 30, 112), (5, 8, 16, 200)])
+def test_state_space_step_of_many_sequences(heads, P, N, seqs):
+    """Steps take other numbers of threads with more sequences and heads (from 297 and from 889 of them on): a sequence's outputs and state
+    are the same, bit for bit, as in a launch of its own."""
+    inner, C = heads * P, heads * P + 2 * N
+    cw, cb, db = rnd(4, C, scale=0.6), rnd(C, seed=1, scale=0.2), rnd(heads, seed=2) - 1
+    a, d, state, ring = -torch.exp(rnd(heads, seed=3)), rnd(heads, seed=4), rnd(seqs, heads, P, N, seed=5), rnd(seqs, 4, C, seed=6)
+    proj = rnd(seqs, 8 * ((2 * inner + 2 * N + heads + 8) // 8), seed=7, dtype=BF16)
+    outs = []
+    for batches in ([range(seqs)], [[s] for s in range(0, seqs, 7)]):
+        st, rg, y = state.clone(), ring.clone(), torch.zeros(seqs, inner, device="cuda")
+        for b in batches:
+            rows = torch.tensor(list(b), device="cuda")
+            out = torch.zeros(len(rows), inner, device="cuda")
+            u, dt = torch.zeros(len(rows), 8 * ((C + 7) // 8), dtype=BF16, device="cuda"), torch.zeros(len(rows), heads, device="cuda")
+            spans = torch.tensor([[i, 1, 9, int(s)] for i, s in enumerate(b)], dtype=torch.int32, device="cuda")
+            k().state_space(proj[rows].contiguous(), cw, cb, db, a, d, st, rg, spans, len(rows), 1, u, dt, out)
+            y[rows] = out
+        outs.append((y[::7], st[::7], rg[::7]))
+    for x, z in zip(*outs):
+        assert torch.equal(x, z)
+
+
 @pytest.mark.parametrize("heads,P,N,groups", [(4, 64, 128, 2), (3, 48, 32, 1), (2, 128, 64, 1), (2, 8, 16, 2), (6, 40, 96, 3)])
 def test_chunked_scan_against_token_scan(heads, P, N, groups):
     """The tensor-core scan keeps 16 bits of every fp32 operand: far closer to the fp32 scan than 16-bit rounding would be.
