@@ -110,7 +110,8 @@ constexpr int kHmCols = 64, kHmSlices = 8, kHmThreads = kHmCols / 2 * kHmSlices;
 // A thread has kHmBatch weights in flight, the first ones before the kernel in front has finished. Tokens of sequences that bring
 // more than `limit` tokens are left alone.
 // Up to 4 tokens, tiles of 4: a quarter of the arithmetic (which is all that is left when the weights come early) and registers for all
-// 64 weights of a 512-deep slice. One token of 32 heads, 512 -> 128: 16.9 us with tiles of 16, 4.3 with tiles of 4.
+// 64 weights of a 512-deep slice. One token of 32 heads, 512 -> 128: 10.0 us with tiles of 16, 4.3 with tiles of 4. Slices of 16 weights and
+// less keep registers for 16, and with them their warps per SM.
 template <int DT, int kHmTok, int kHmBatch>
 __global__ void __launch_bounds__(kHmThreads)
 head_matmul_kernel(const void* __restrict__ x, int64_t ld_x, int in_width, const void* __restrict__ w, void* __restrict__ out,
@@ -260,7 +261,11 @@ extern "C" int hds_head_matmul(const void* x, int64_t ld_x, int in_width, const 
                                      out_width, tok_seq, spans, limit, T, K, N, copy));                                        \
     } while (0)
     if (tok == 4) {
-        if (dtype == 0) HDS_HM(0, 4, 64);
+        if (K <= 16 * kHmSlices) {
+            if (dtype == 0) HDS_HM(0, 4, 16);
+            else if (dtype == 1) HDS_HM(1, 4, 16);
+            else HDS_HM(2, 4, 16);
+        } else if (dtype == 0) HDS_HM(0, 4, 64);
         else if (dtype == 1) HDS_HM(1, 4, 64);
         else HDS_HM(2, 4, 32);
     } else {
