@@ -559,10 +559,16 @@ static int launch_pair(const CUtensorMap& tq, const CUtensorMap& tkv, const Pref
 }
 
 // Two heads of a group per CTA: head_dim 128, an even group, no ALiBi, no KV split, and at least as many pairs as SMs (at 12 items of
-// 128 tokens x 32 heads, 192 pairs, 28.2 -> 26.9 us; with fewer, one head per CTA keeps more SMs busy). Not where 64-key tiles are asked for.
+// 128 tokens x 32 heads, 192 pairs, 28.2 -> 26.9 us; with fewer, one head per CTA keeps more SMs busy). Sigmoid weights and bounded
+// scores are bound by their exponentials and quotients, a pair saves them 5 - 15 % only, so that a second wave that is nearly empty
+// costs more: 160 pairs of 30 tokens behind 2000, sigmoid 90.5 us by head and 105.7 by pairs, bounded 130.2 and 148.1, softmax 86.5 and
+// 73.0. They take pairs from half a second wave on: 256 pairs of 2048 tokens behind 6000 393.8 and 359.2, 567.3 and 535.5 (the first 2048
+// tokens alone, whose items are unequal, 89.3 and 90.7, 120.0 and 126.4). Not where 64-key tiles are asked for.
 static bool use_pair(const PrefillArgs& a, int head_dim, int n_items) {
+    const int64_t pairs = static_cast<int64_t>(n_items) * (a.n_q_heads / 2);
+    const bool plain = a.sigmoid_bias == nullptr && a.cap_log2 <= 0.0f;
     return !prefill64_enabled() && head_dim == 128 && (a.n_q_heads / a.n_kv_heads) % 2 == 0 && a.alibi == nullptr && a.n_splits == 1 &&
-           static_cast<int64_t>(n_items) * (a.n_q_heads / 2) >= sm_count();
+           (plain ? pairs >= sm_count() : 2 * pairs >= 3 * sm_count());
 }
 
 template <int D, bool kBf16, bool kPacked, int kWeights>

@@ -741,6 +741,20 @@ print([e.key for e in p.key_averages()])
     assert kernel in res.stdout
 
 
+def prefill_of(items, **kw):
+    q, cache, tables, its = build_paged_problem([(64, 64)] * items, 16, 4, 128, 64)
+    if "sigmoid" in kw:
+        kw = dict(sigmoid_bias=torch.full((16, ), -3.0, device="cuda"))
+    K().paged_attention_prefill(q, torch.empty_like(q), cache, tables, torch.tensor(its, dtype=torch.int32, device="cuda"), items, 16, 4, 128, 64, 0.09, **kw)
+
+
+def test_attention_pair_rule():
+    """Pairs of heads from one per SM on, weights with quotients from three for two SMs on: the kernel that runs, at 8 pairs an item."""
+    cases = [("18", "prefill"), ("19", "pair"), ("27, softcap=4.0", "prefill"), ("28, softcap=4.0", "pair"), ("27, sigmoid=1", "prefill"), ("28, sigmoid=1", "pair")]
+    for names, (args, kernel) in zip(kernels_of([f"t.prefill_of({a})" for a, _ in cases]), cases):
+        assert f"paged_attn_{kernel}_kernel" in names, args
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("opts", ["plain", "window", "keep", "sink", "sigmoid", "softcap"])
 @pytest.mark.parametrize("n_q_heads,n_kv,bs", [(16, 4, 64), (12, 2, 16), (32, 1, 128)])
