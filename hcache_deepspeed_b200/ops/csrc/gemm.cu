@@ -137,10 +137,9 @@ static bool skinny_enabled() {
     return on != 0;
 }
 
-template <int NT, int EPI, bool kBf16, bool kGrouped = false>
-static int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid,
-                              cudaStream_t stream) {
-    auto kern = gemm_skinny_kernel<NT, EPI, kBf16, false, kGrouped>;
+template <int NT, int EPI, bool kBf16, bool kGrouped, bool kMeet>
+static int launch_skinny_as(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid, cudaStream_t stream) {
+    auto kern = gemm_skinny_kernel<NT, EPI, kBf16, false, kGrouped, kMeet>;
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -149,9 +148,16 @@ static int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, cons
                                             static_cast<int>(skinny_smem_bytes(NT, kGrouped))));
         configured[dev & 63] = true;
     }
-    HDS_CHECK_CUDA(launch_kernel_cluster(kern, EPI == EPI_RED_F32 || kGrouped ? 1 : a.splits, dim3(grid), dim3(kGemmThreads),
-                                         skinny_smem_bytes(NT, kGrouped), stream, tw, tx, a));
+    HDS_CHECK_CUDA(launch_kernel_cluster(kern, kMeet ? a.splits : 1, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT, kGrouped), stream,
+                                         tw, tx, a));
     return HDS_OK;
+}
+
+template <int NT, int EPI, bool kBf16, bool kGrouped = false>
+static int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid, cudaStream_t stream) {
+    if constexpr (EPI != EPI_RED_F32 && !kGrouped)
+        if (a.splits > 1) return launch_skinny_as<NT, EPI, kBf16, false, true>(tw, tx, a, grid, stream);
+    return launch_skinny_as<NT, EPI, kBf16, kGrouped, false>(tw, tx, a, grid, stream);
 }
 
 template <int EPI, bool kBf16, bool kGrouped = false>

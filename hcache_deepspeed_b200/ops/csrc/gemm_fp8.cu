@@ -360,9 +360,9 @@ extern "C" int hds_gemm_fp8(const void* Aq, int64_t lda, const float* a_scale, c
 // ---- decode-size M: the feature-major weight-streaming kernel (gemm_skinny.cuh) with E4M3 operands --------------
 namespace hds {
 
-template <int NT, int EPI, bool kBf16>
-static int launch_skinny_fp8_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid, cudaStream_t stream) {
-    auto kern = gemm_skinny_kernel<NT, EPI, kBf16, true>;
+template <int NT, int EPI, bool kBf16, bool kMeet>
+static int launch_skinny_fp8_as(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid, cudaStream_t stream) {
+    auto kern = gemm_skinny_kernel<NT, EPI, kBf16, true, false, kMeet>;
     static bool configured[64] = {false};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -371,8 +371,15 @@ static int launch_skinny_fp8_inst(const CUtensorMap& tw, const CUtensorMap& tx, 
                                             static_cast<int>(skinny_smem_bytes(NT))));
         configured[dev & 63] = true;
     }
-    HDS_CHECK_CUDA(launch_kernel_cluster(kern, EPI == EPI_RED_F32 ? 1 : a.splits, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT), stream, tw, tx, a));
+    HDS_CHECK_CUDA(launch_kernel_cluster(kern, kMeet ? a.splits : 1, dim3(grid), dim3(kGemmThreads), skinny_smem_bytes(NT), stream, tw, tx, a));
     return HDS_OK;
+}
+
+template <int NT, int EPI, bool kBf16>
+static int launch_skinny_fp8_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyArgs& a, int grid, cudaStream_t stream) {
+    if constexpr (EPI != EPI_RED_F32)
+        if (a.splits > 1) return launch_skinny_fp8_as<NT, EPI, kBf16, true>(tw, tx, a, grid, stream);
+    return launch_skinny_fp8_as<NT, EPI, kBf16, false>(tw, tx, a, grid, stream);
 }
 
 template <int EPI, bool kBf16>

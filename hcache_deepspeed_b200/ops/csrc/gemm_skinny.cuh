@@ -35,7 +35,7 @@ __host__ __device__ constexpr size_t skinny_smem_bytes(int nt, bool grouped = fa
     return static_cast<size_t>(skinny_stages(nt, grouped)) * (kSkinnyBF * kGemmBK * 2 + nt * kGemmBK * 2) + 256 + 1024;
 }
 
-// K splits of a decode GEMM of n_tiles feature tiles. Measured (profiles/kernel_bench_decode_gemm.jsonl): fill the resident slots once;
+// K splits of a decode GEMM of n_tiles feature tiles. Measured: fill the resident slots once;
 // past one full wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4
 // splits). At most 8, the size of a portable cluster; a count that the caller gives is held to that where the splits meet in one (`clusters`),
 // and to the K blocks where they add up in memory. A cluster needs its slots in one GPC, so that some stay empty: where the splits
@@ -157,7 +157,8 @@ __device__ __forceinline__ void cluster_sync() {
 // to the routing kernels before it only, so nothing is requested ahead of them. Every expert's weights are streamed once: the
 // token-major kernel's 256-wide tiles are too few for that (8 tokens x top 2 of 16 experts of 2048 x 2688: 35 us up and 26 us down,
 // 3.6 TB/s).
-template <int NT, int EPI, bool kBf16, bool kFp8 = false, bool kGrouped = false>
+// kMeet: the K splits of a store / gated tile, a cluster. A form of its own, because what it adds costs unsplit tiles up to 7 %.
+template <int NT, int EPI, bool kBf16, bool kFp8 = false, bool kGrouped = false, bool kMeet = false>
 __global__ void __launch_bounds__(kGemmThreads, skinny_occupancy(NT, kGrouped))
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const SkinnyArgs args) {
@@ -183,9 +184,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int n_tiles = (args.N + kSkinnyBF - 1) / kSkinnyBF;
     const int kb_total = (args.K + KB - 1) / KB;
     // (kGrouped: sp is the place of the expert; else the K split, whose CTAs are neighbours where they are a cluster)
-    const bool meet = EPI != EPI_RED_F32 && !kGrouped && args.splits > 1;
-    const int n_t = meet ? static_cast<int>(blockIdx.x) / args.splits : static_cast<int>(blockIdx.x) % n_tiles;
-    const int sp = meet ? static_cast<int>(blockIdx.x) % args.splits : static_cast<int>(blockIdx.x) / n_tiles;
+    static_assert(!kMeet || (EPI != EPI_RED_F32 && !kGrouped), "the other forms have nothing to meet for");
+    const int n_t = kMeet ? static_cast<int>(blockIdx.x) / args.splits : static_cast<int>(blockIdx.x) % n_tiles;
+    const int sp = kMeet ? static_cast<int>(blockIdx.x) % args.splits : static_cast<int>(blockIdx.x) / n_tiles;
     const int kb0 = kGrouped ? 0 : sp * args.kb_per_split;
     const int kb1 = min(kb_total, kb0 + args.kb_per_split);
     const uint32_t w_tx = args.w_tx_bytes ? args.w_tx_bytes : W_BYTES;
@@ -307,7 +308,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         } else {
             constexpr bool kGated = EPI == EPI_GATED;
-            if (!meet) {
+            if constexpr (!kMeet) {
                 skinny_finalize<NT, kBf16, kGated>(args, n, lane, v, 0, 1, x_row);
             } else {      // (the stages are free: every product has been read out of them)
                 float* part = reinterpret_cast<float*>(smem) + quad * 32 + lane;
@@ -317,26 +318,24 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
     }
-    if constexpr (EPI != EPI_RED_F32 && !kGrouped) {
-        if (meet) {
-            __syncwarp();
-            cluster_sync();       // every split's sums are there
-            if (warp >= 2) {
-                constexpr int C = 4;      // tokens at a time
-                const uint32_t quad = warp & 3;
-                const int n = n_t * kSkinnyBF + static_cast<int>(quad * 32 + lane);
-                const float* part = reinterpret_cast<const float*>(smem) + quad * 32 + lane;
-                for (int t0 = sp; t0 < args.M; t0 += C * args.splits) {
-                    float v[C] = {};
-                    for (int s = 0; s < args.splits; ++s)
+    if constexpr (kMeet) {
+        __syncwarp();
+        cluster_sync();       // every split's sums are there
+        if (warp >= 2) {
+            constexpr int C = 4;      // tokens at a time
+            const uint32_t quad = warp & 3;
+            const int n = n_t * kSkinnyBF + static_cast<int>(quad * 32 + lane);
+            const float* part = reinterpret_cast<const float*>(smem) + quad * 32 + lane;
+            for (int t0 = sp; t0 < args.M; t0 += C * args.splits) {
+                float v[C] = {};
+                for (int s = 0; s < args.splits; ++s)
 #pragma unroll
-                        for (int i = 0; i < C; ++i) v[i] += cluster_load(part + min(t0 + i * args.splits, args.M - 1) * kSkinnyBF, s);
-                    skinny_finalize<C, kBf16, EPI == EPI_GATED>(args, n, lane, v, t0, args.splits);
-                }
+                    for (int i = 0; i < C; ++i) v[i] += cluster_load(part + min(t0 + i * args.splits, args.M - 1) * kSkinnyBF, s);
+                skinny_finalize<C, kBf16, EPI == EPI_GATED>(args, n, lane, v, t0, args.splits);
             }
-            __syncwarp();
-            cluster_sync();       // nobody leaves while its sums are read
         }
+        __syncwarp();
+        cluster_sync();       // nobody leaves while its sums are read
     }
 
     tc_fence_before();
