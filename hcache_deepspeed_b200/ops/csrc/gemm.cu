@@ -168,6 +168,24 @@ static int launch_skinny_nt(int nt, const CUtensorMap& tw, const CUtensorMap& tx
     return launch_skinny_inst<64, EPI, kBf16, kGrouped>(tw, tx, a, grid, stream);
 }
 
+// More than 32 tokens of short rows and more feature tiles than run at once: a tile's 64-column epilogue weighs more than its weights. 64 tokens,
+// token-major against feature-major: 50272 x 2048 39.1 and 43.0 us, 128256 x 2048 84.9 and 92.2; 57344 x 4096 92.9 and 82.7, 151936 x 4096
+// 208.4 and 199.1.
+static bool short_rows_past_a_wave(int M, int N, int K) {
+    return M > 32 && (N + kSkinnyBF - 1) / kSkinnyBF > sm_count() * skinny_occupancy(64) && K < 4096;
+}
+
+// Plain stores of 17 to 64 tokens that stay with the token-major kernel: those above, and where its tiles nearly fill the chip in one wave,
+// so that more of them in flight gain little over what the splits' meeting costs. Token-major against feature-major: 14336 x 2048 32 tokens
+// 14.6 and 15.3 us, 64 tokens 14.7 and 17.7; 14336 x 8192 64 tokens 45.5 and 48.5; 12288 x 2048 64 tokens 14.9 and 17.0; but 14336 x 4096 17
+// tokens 25.3 and 24.4, 12288 x 4096 33 tokens 24.3 and 23.4, 14336 x 14336 64 tokens 73.3 and 72.2, 10240 x 2048 33 tokens 13.9 and 12.5.
+static bool store_token_major(int M, int N, int K) {
+    if (short_rows_past_a_wave(M, N, K)) return true;
+    const int n_tiles = (N + kSkinnyBF - 1) / kSkinnyBF, sms = sm_count();
+    if (n_tiles > sms || n_tiles * 10 <= sms * 6) return false;
+    return n_tiles * 10 > sms * 7 ? K <= (M > 32 ? 8192 : 2048) : M > 32 && K <= 2048;
+}
+
 // One CTA per (128-feature tile, K split); splits fill the resident slots (SMs x CTAs per SM) once. No scratch.
 static int launch_skinny(int epi, bool bf16, const void* X, int64_t ldx, const void* W, int64_t ldw, int M, int N,
                          int K, int act, const void* bias, void* out, int64_t ldo, float* accum, int64_t ld_accum,
@@ -289,12 +307,12 @@ extern "C" int hds_gemm(const void* A, int64_t lda, const void* W, int64_t ldw, 
     HDS_REQUIRE(epilogue == EPI_STORE || epilogue == EPI_GATED, "hds_gemm: epilogue must be 0 (store) or 1 (gated)");
     HDS_REQUIRE(dtype == 0 || dtype == 1, "hds_gemm: dtype must be 0 (bf16) or 1 (fp16)");
     HDS_REQUIRE(epilogue != EPI_GATED || (N % 2 == 0), "hds_gemm: gated epilogue needs an even N");
-    // Up to 64 tokens the feature-major kernel streams the weights. Plain stores, 64 tokens, token-major against it: 10240 x 8192 40.8
-    // and 32.7 us, 32000 x 8192 90.1 and 83.4, 12288 x 4096 23.5 and 23.3, 6144 x 4096 20.7 and 14.5, 2048 x 2048 9.9 and 7.0; at 17
-    // tokens 40.6 and 29.4, 23.1 and 20.4, 8.2 and 5.3. The gated MLP-1 at 17 - 64 tokens only where it is wide: a tensor-parallel
-    // rank's 2752 features were 1.3 x faster in the token-major kernel.
-    if (M <= 64 && ldw >= 0 &&
-        (bn == -1 || (bn == 0 && skinny_enabled() && (M <= 16 || epilogue == EPI_STORE || N >= 8192))))
+    // Up to 64 tokens the feature-major kernel streams the weights. Plain stores, 64 tokens, token-major against it: 10240 x 8192 42.5
+    // and 34.4 us, 32000 x 8192 91.5 and 86.1, 6144 x 4096 21.3 and 15.2, 22016 x 4096 49.3 and 37.1; at 17 tokens 41.8 and 30.5, 90.5 and
+    // 82.2, 17.0 and 12.5, 59.3 and 34.4. The gated MLP-1 at 17 - 64 tokens only where it is wide: a tensor-parallel rank's 2752 features
+    // were 1.3 x faster in the token-major kernel.
+    if (M <= 64 && ldw >= 0 && (bn == -1 || (bn == 0 && skinny_enabled() &&
+                                             (M <= 16 || (epilogue == EPI_STORE ? !store_token_major(M, N, K) : N >= 8192)))))
         return launch_skinny(epilogue, dtype == 0, A, lda, W, ldw, M, N, K, act, bias, out, ldo, nullptr, 0, splits, static_cast<cudaStream_t>(stream));
     // measured (profiles/kernel_bench_gemm_2sm.txt): with at least one full wave of 256 x 256 pair tiles the
     // cta_group::2 kernel is 1.10-1.20x the single-CTA kernel and level with cuBLAS
@@ -348,7 +366,7 @@ extern "C" int hds_gemm_accum(const void* A, int64_t lda, const void* W, int64_t
     // 4.8, 512 x 8192 5.5 and 7.0, 1024 x 4096 5.5 and 4.9, 1024 x 8192 7.7 and 7.8, 4096 x 4096 9.7 and 8.6. 64 tokens, 1536 x 4096 6.8
     // token-major, 2048 x 4096 7.4 and 7.4, 2048 x 8192 10.2 and 11.0, 2752 x 8192 12.3 and 12.8, 4096 x 8192 16.0 and 15.5, 8192 x 28672
     // 79.1 and 73.3.
-    const bool wide = M <= 16 || (M <= 32 ? N >= 1024 : N >= (K <= 4096 ? 2048 : 4096));
+    const bool wide = M <= 16 || (M <= 32 ? N >= 1024 : N >= (K <= 4096 ? 2048 : 4096) && !short_rows_past_a_wave(M, N, K));
     if (M <= 64 && ldw >= 0 && red_mode == 0 && n_targets == 1 && (bn == -1 || (bn == 0 && skinny_enabled() && wide)))
         return launch_skinny(EPI_RED_F32, dtype == 0, A, lda, W, ldw, M, N, K, 0, bias, nullptr, 0, accum_ptrs[0],
                              ld_accum, splits, static_cast<cudaStream_t>(stream));

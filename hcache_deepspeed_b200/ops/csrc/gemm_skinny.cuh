@@ -39,7 +39,10 @@ __host__ __device__ constexpr size_t skinny_smem_bytes(int nt, bool grouped = fa
 // past one full wave of tiles, split until the waves are >= 80 % full (448 tiles of a 57344-wide MLP-1: 5.25 -> 5.66 TB/s at 4
 // splits). At most 8, the size of a portable cluster; a count that the caller gives is held to that where the splits meet in one (`clusters`),
 // and to the K blocks where they add up in memory. A cluster needs its slots in one GPC, so that some stay empty: where the splits
-// meet in one, they fill no more than 87 % (96 tiles x 3 of 296 slots: 27.7 us at 17 tokens of 12288 x 4096, 20.4 us in 2).
+// meet in one, they fill no more than 87 % (96 tiles x 3 of 296 slots: 27.7 us at 17 tokens of 12288 x 4096, 20.4 us in 2). Past one
+// wave clusters of more than 16 tokens are slower than the empty slots of a last wave (64 tokens, unsplit and in 2 or 3: 57344 x 8192 148.3
+// and 170.3 us, 57344 x 2048 45.2 and 71.2, 50272 x 4096 77.3 and 82.4), but for long rows on a wave less than 60 % full (17 tokens of
+// 43008 x 8192: 124.2 and 117.7).
 inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms, bool clusters) {
     int splits = want;
     if (want <= 0) {
@@ -57,6 +60,8 @@ inline int skinny_splits(int n_tiles, int kb_total, int nt, int want, int sms, b
                     break;
                 }
             }
+            const int64_t waves = (n_tiles + slots - 1) / slots;
+            if (clusters && nt > 16 && !(kb_total >= 128 && static_cast<int64_t>(n_tiles) * 100 < waves * slots * 60)) splits = 1;
         }
         if (splits > kb_total / 4) splits = kb_total / 4;
     }

@@ -741,6 +741,28 @@ print([e.key for e in p.key_averages()])
     assert kernel in res.stdout
 
 
+STORE_RULE = [(16, 57344, 512, "gemm_skinny"), (17, 14336, 2048, "gemm_tn"), (17, 14336, 2056, "gemm_skinny"), (33, 14336, 8192, "gemm_tn"), (33, 13312, 2048, "gemm_tn"),
+              (64, 12288, 2048, "gemm_tn"), (64, 11264, 2048, "gemm_skinny"), (33, 12288, 2056, "gemm_skinny"), (64, 18944, 2048, "gemm_tn"), (64, 18952, 2048, "gemm_skinny"),
+              (33, 37888, 2048, "gemm_skinny"), (33, 37896, 2048, "gemm_tn"), (32, 37896, 2048, "gemm_skinny"), (64, 37896, 4096, "gemm_skinny")]
+
+
+def test_gemm_store_rule():
+    """Plain stores of decode sizes on both sides of each line of the rule: the kernel that runs."""
+    ran = kernels_of([f"t.K().gemm(t.rand({M}, {K_}), t.rand({N}, {K_}), out=t.rand({M}, {N}))" for M, N, K_, _ in STORE_RULE])
+    for names, case in zip(ran, STORE_RULE):
+        assert case[3] in names, case
+
+
+@pytest.mark.parametrize("M,N,K_,gated", [(33, 37896, 256, False), (64, 37896, 256, True), (17, 43008, 8192, False), (64, 13320, 512, False), (40, 57344, 4096, True)])
+def test_gemm_past_a_wave(M, N, K_, gated):
+    """More feature tiles than run at once, split and unsplit, and widths around the rule: against the product in fp32."""
+    torch.manual_seed(M + N)
+    a, w, b = rand(M, K_), rand(N, K_, scale=K_ ** -0.5), rand(N)
+    out = K().gemm(a, w, bias=b, act=3 if gated else 0, gated=gated)
+    want = ref.gemm(a, w, bias=b, act=3 if gated else 0, gated=gated, out_dtype=torch.float32)
+    torch.testing.assert_close(out.float(), want, **tol(torch.bfloat16))
+
+
 def prefill_of(items, **kw):
     q, cache, tables, its = build_paged_problem([(64, 64)] * items, 16, 4, 128, 64)
     if "sigmoid" in kw:
