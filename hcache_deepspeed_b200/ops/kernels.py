@@ -487,6 +487,13 @@ def paged_attention_prefill(q: torch.Tensor, out: torch.Tensor, kv_cache_layer: 
 MOE_FEW = 64
 
 
+def _moe_few(choices: int, K: int, gated: bool) -> bool:
+    """The token tile has room for all choices at one expert. Gated, and more than 32 wide, its epilogue costs more than a short weight row
+    saves: 64 choices of 64 experts of 2816 x 1024 55.1 us token-major and 66.0 feature-major, 128 of 1536 x 768 36.2 and 43.7, 16 of 2816 x
+    2048 46.1 and 47.2; 64 of 7168 x 4096 486 and 428. Plain ones gain at all sizes (64 of 2048 x 1408 56.5 and 55.5)."""
+    return 0 < choices <= MOE_FEW and (not gated or choices <= 32 or K >= 4096)
+
+
 def moe_padded_rows(n_tokens: int, n_experts: int, top_k: int) -> int:
     """Row capacity of the scattered activation buffer (each expert's range is padded to 128 rows)."""
     return int(native.cuda_lib().hds_moe_padded_rows(n_tokens, n_experts, top_k))
@@ -523,7 +530,7 @@ def moe_scatter(x: torch.Tensor, xs: torch.Tensor, expert_ids: torch.Tensor, off
 def moe_gemm(a: torch.Tensor, w_stacked: torch.Tensor, pad_off: torch.Tensor, n_experts: int, out: torch.Tensor,
              act: int = ACT_IDENTITY, gated: bool = False, limit: float = 0.0, choices: int = 0) -> torch.Tensor:
     """Grouped GEMM: rows of ``a`` in expert e's range times ``w_stacked[e*N:(e+1)*N]``ᵀ (``w_stacked``: [E*N, K]). ``choices`` (0: not
-    known): how many rows live in all; up to 64 of them take the kernel that streams the weights (see ``MOE_FEW``)."""
+    known): how many rows live in all; few of them take the kernel that streams the weights."""
     _check_2d(a, "a")
     _check_2d(out, "out")
     rows, K = a.shape
@@ -533,7 +540,7 @@ def moe_gemm(a: torch.Tensor, w_stacked: torch.Tensor, pad_off: torch.Tensor, n_
         return _gemm_f32(a, w_stacked, out, EPI_GATED if gated else EPI_STORE, act, limit, pad_off, n_experts)
     if act == ACT_SWIGLU_CLAMPED:
         native.check(native.cuda_lib().hds_gemm_next_act_limit(limit), "hds_gemm_next_act_limit")
-    if 0 < choices <= MOE_FEW:
+    if _moe_few(choices, K, gated):
         rc = native.cuda_lib().hds_moe_gemm_few(_p(a), a.stride(0), _p(w_stacked), w_stacked.stride(0), _p(pad_off), n_experts, choices,
                                                 choices, rows, N, K, _dt(a), EPI_GATED if gated else EPI_STORE, act, _p(out),
                                                 out.stride(0), _stream())

@@ -770,6 +770,19 @@ def prefill_of(items, **kw):
     K().paged_attention_prefill(q, torch.empty_like(q), cache, tables, torch.tensor(its, dtype=torch.int32, device="cuda"), items, 16, 4, 128, 64, 0.09, **kw)
 
 
+def experts_of(choices, K_, gated):
+    x, w, pad = torch.zeros(256, K_, dtype=torch.bfloat16, device="cuda"), rand(256, K_), torch.tensor([0, 128, 256], dtype=torch.int32, device="cuda")
+    K().moe_gemm(x, w, pad, 2, torch.empty(256, 64 if gated else 128, dtype=torch.bfloat16, device="cuda"), gated=gated, choices=choices)
+
+
+def test_experts_rule():
+    """Expert products of a decode step: the kernel by choices, inner size and form."""
+    cases = [("0, 128, False", "gemm_tn"), ("64, 128, False", "gemm_skinny"), ("65, 128, False", "gemm_tn"), ("32, 128, True", "gemm_skinny"), ("33, 4088, True", "gemm_tn"),
+             ("64, 4096, True", "gemm_skinny")]
+    for names, (args, kernel) in zip(kernels_of([f"t.experts_of({a})" for a, _ in cases]), cases):
+        assert kernel in names, args
+
+
 def test_attention_pair_rule():
     """Pairs of heads from one per SM on, weights with quotients from three for two SMs on: the kernel that runs, at 8 pairs an item."""
     cases = [("18", "prefill"), ("19", "pair"), ("27, softcap=4.0", "prefill"), ("28, softcap=4.0", "pair"), ("27, sigmoid=1", "prefill"), ("28, sigmoid=1", "pair")]
