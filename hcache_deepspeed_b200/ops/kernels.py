@@ -119,8 +119,8 @@ def gemm(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, 
          gated: bool = False, out: Optional[torch.Tensor] = None, bn: int = 0, splits: int = 0,
          workspace: Optional[torch.Tensor] = None, limit: float = 0.0) -> torch.Tensor:
     """``out = epilogue(a @ w.T + bias)`` on the tcgen05 GEMM. ``gated``: interleaved (gate, up) columns.
-    ``workspace`` (zero-initialised uint8 scratch) enables split-K for decode-size M. ``limit``: the bound of
-    ``ACT_SWIGLU_CLAMPED``. fp32 operands take the plain fp32 kernel."""
+    ``workspace`` (zero-initialised uint8 scratch): lets the token-major kernel split K for decode-size M; up to 64 tokens the
+    feature-major one splits without (``splits=1``: none does). ``limit``: the bound of ``ACT_SWIGLU_CLAMPED``. fp32 operands take the plain fp32 kernel."""
     _check_2d(a, "a")
     M, K = a.shape
     N = w.shape[0]
@@ -593,8 +593,8 @@ def gemm_fp8(aq: torch.Tensor, a_scale: torch.Tensor, wq: torch.Tensor, w_scale:
              workspace: Optional[torch.Tensor] = None, splits: int = 0, w_fmt: int = 0) -> torch.Tensor:
     """``out = epilogue((aq @ wq.T) * a_scale[:, None] * w_scale[None, :] + bias)`` with E4M3 operands on
     ``tcgen05.mma.kind::f8f6f4`` (fp32 accumulation in TMEM). ``aq``: [M, K] uint8, ``wq``: [N, K] uint8.
-    M <= 64 with ``bn == 0`` takes the feature-major weight-streaming kernel (split-K through ``workspace``, a zeroed
-    uint8 buffer of at least :func:`gemm_fp8_skinny_workspace_bytes`)."""
+    M <= 64 with ``bn == 0`` takes the feature-major weight-streaming kernel, which splits K for a caller that gives a ``workspace`` of
+    at least :func:`gemm_fp8_skinny_workspace_bytes` (it is not written: the parts meet in a cluster)."""
     _check_2d(aq, "aq")
     _check_2d(wq, "wq")
     _check_2d(out, "out")

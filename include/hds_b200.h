@@ -31,9 +31,10 @@ const char* hds_last_error(void);
  * 3 silu, 4 gelu-tanh.  bn: tile width override (0 = heuristic; -1 = force the
  * feature-major weight-streaming kernel of gemm_skinny.cuh, M <= 64 only).
  * Ref: core_ops/blas_kernels/blas.h:31-136 + bias_activations + gated_activations.
- * Split-K (decode-size M <= 128): pass a zero-initialised scratch buffer of at least
- * hds_gemm_splitk_workspace_bytes(M, N) bytes; partial sums meet there and the last split applies the
- * epilogue and leaves the buffer zeroed again. splits: 0 = heuristic, 1 = off. Without scratch: no split. */
+ * Split-K (decode-size M <= 128), splits: 0 = heuristic, 1 = off. The feature-major kernel (M <= 64) splits without scratch, in
+ * up to 8 parts that meet in a cluster in a fixed order. The token-major kernel (all of 65..128, some of 17..64) wants a
+ * zero-initialised scratch of at least hds_gemm_splitk_workspace_bytes(M, N) bytes, where partial sums meet in the order of
+ * their arrival; the last split applies the epilogue and leaves it zeroed again. Without scratch it does not split. */
 int64_t hds_gemm_splitk_workspace_bytes(int M, int N);
 int hds_gemm(const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K, int dtype, int epilogue,
              int act, const void* bias, void* out, int64_t ldo, int bn, int splits, void* splitk_ws,
@@ -63,7 +64,7 @@ int hds_restore_kv_proj(const void* latents, int64_t ld_latents, const void* w_k
  * calling process: symmetric memory / CUDA IPC / cuMemMap peer mapping). The kernel's TMA producer reads every tile
  * straight from the owning peer over NVLink; each rank projects all T tokens onto its own KV heads.
  * latent_ptrs is a HOST array; rows_per_peer is a multiple of 128. The caller orders the launch after every peer's
- * buffer is filled (device barrier). Ref: SURVEY 2.8 "(new) restore under TP" — absent in the reference. */
+ * buffer is filled (device barrier). No reference counterpart: restore under tensor parallelism is absent there. */
 int hds_restore_kv_proj_peers(const void* const* latent_ptrs, int n_peers, int rows_per_peer, int64_t ld_latents,
                               const void* w_kv, int64_t ldw, int T, int H, int dtype, const void* bias_kv,
                               void* kv_cache_layer, const int32_t* tok_pos, const int32_t* tok_slot,
@@ -208,7 +209,7 @@ int hds_paged_attention_splitkv(const void* q, void* out, const void* kv_cache_l
                                 int dtype, void* stream);
 
 /* The same for query heads that share their keys (any group size is taken): mma.sync over strips of 16 keys, weights split into
- * two 16-bit parts; scratch as above. */
+ * two 16-bit parts (2^-17 of a weight in bf16; fp16 keeps 2^-22 down to weights of 2^-17); scratch as above. */
 int hds_paged_attention_group(const void* q, void* out, const void* kv_cache_layer, int64_t num_blocks,
                               const int32_t* block_tables, int max_blocks_per_seq, const hds_attn_item* items,
                               int n_items, int rows_per_item, int n_q_heads, int n_kv_heads, int head_dim,
@@ -349,8 +350,9 @@ int hds_gemm_fp8(const void* Aq, int64_t lda, const float* a_scale, const void* 
                  int bn, void* stream);
 
 /* Decode-size (M <= 64) E4M3 GEMM on the feature-major weight-streaming kernel: epilogue 0 store / 1 gated (into out) or
- * 2 fp32 accumulate (accum[m, n] += ..., bias added once). Split-K for store / gated needs a zeroed scratch of
- * hds_gemm_fp8_skinny_workspace_bytes(M, N) bytes (left zeroed); splits 0 = auto. lda / ldw in bytes. */
+ * 2 fp32 accumulate (accum[m, n] += ..., bias added once). Store / gated split K only for a caller that brings a scratch of
+ * hds_gemm_fp8_skinny_workspace_bytes(M, N) bytes: the parts meet in a cluster, so that it is neither read nor written, but a
+ * caller without one keeps unsplit sums. splits 0 = auto. lda / ldw in bytes. */
 int64_t hds_gemm_fp8_skinny_workspace_bytes(int M, int N);
 int hds_gemm_fp8_skinny(const void* Aq, int64_t lda, const float* a_scale, const void* Wq, int64_t ldw, const float* w_scale,
                         int M, int N, int K, int out_dtype, int epilogue, int act, const void* bias, void* out, int64_t ldo,
