@@ -15,8 +15,8 @@
 // in the neighbouring lane), fp32 accumulate into the pending residual delta (split-K needs no meeting there).
 // The K splits of a store / gated tile are a cluster (up to 8): each leaves its sums in its shared memory, behind the cluster's barrier
 // CTA r adds up the tokens r, r + splits, ... of all of them and stores those. Through an fp32 scratch in global memory, with
-// atomic sums and tickets, the end of a tile took 3 - 4 us more: in a decode step of one token, 12288 x 4096 in 4 splits 20.5 us
-// so and 16.5 us now, the gated 22016 x 4096 in 2 splits 31.4 and 27.6 us (6.5 TB/s).
+// atomic sums and tickets, the end of a tile took 1 - 2 us more: one token, weights read from memory (300 MB of them in turn),
+// 12288 x 4096 19.8 us so and 17.6 now, the gated 22016 x 4096 31.4 and 29.0 us (6.2 TB/s), 2048 x 2048 6.5 and 4.5.
 //
 // Role in the reference: the cuBLAS GEMMs of a decode step (core_ops/blas_kernels/blas.h:31-136) plus the
 // bias / gated activation kernels that follow them.

@@ -105,7 +105,7 @@ int hds_norm_next_fp8(void* q, int64_t ldq, float* scales);
  * hds_tp_ctx_create: pad_ptrs is a HOST array [n_ranks] of this rank's mappings of every rank's pad
  * (pad_ptrs[rank] = the local one). Returns a context id >= 0, or a negative error.
  * hds_tp_arm: attaches a wait and / or a signal to the NEXT kernel this host thread launches through hds_gemm,
- * hds_gemm_accum, hds_gemm_2sm, hds_gemm_fp8, hds_gemm_fp8_skinny, hds_moe_gemm, hds_qkv_rope_proj,
+ * hds_gemm_accum, hds_gemm_2sm, hds_gemm_fp8, hds_gemm_fp8_skinny, hds_moe_gemm, hds_moe_gemm_few, hds_qkv_rope_proj,
  * hds_restore_kv_proj, hds_quantize_fp8_rows (wait only) or hds_p2p_gather_rows (wait only):
  *   wait   - the kernel's TMA producer (or every CTA) acquires all ranks' flags before it reads activations that
  *            the peers wrote into this GPU's buffer (all-gather -> GEMM);
