@@ -588,6 +588,7 @@ N_SM = 148
 MAX_DECODE_SPLITS = 16
 MAX_PREFILL_SPLITS = 16
 MAX_LATENT_SPLITS = 64
+NARROW_LATENT = 256     # values of a latent up to which more than 16 splits have two tiles each
 MAX_SMALL_ROWS = 8      # query rows per item and KV head that the kernels of few rows take
 
 
@@ -685,13 +686,17 @@ def latent_splits(n_items: int, item_tokens: int, heads: int, rank: int, width: 
     """KV splits of the latent attention kernel: one wave of CTAs at most, at least one tile each. The few-rows kernel (128-key tiles) takes
     up to 64, merged by a kernel of its own (one token, 32 heads, 4096 cached rows: 16 splits of up to three tiles take 28.6 us with
     the merge, a tile each 22.1): a power of two, so that a growing context does not ask for another graph with every tile; splits without a tile
-    leave at once."""
+    leave at once. A tile of a narrow latent takes little longer than merging its split, so that more than 16 splits get two tiles each (one
+    token, 8 heads of 128 values: 4096 rows 12.5 us in 16 splits and 13.6 in 32, 8000 rows 16.0 in 16 and 18.6 in 63; 20 heads of 256: 8000 rows
+    21.5 in 16 and 21.8 in 63; 512 values: 34.8 and 28.5)."""
     from .kernels import latent_attention_ctas
     ctas, tile = latent_attention_ctas(item_tokens, heads, rank, width)
     tiles = max(1, -(-(min(max_kv_len, window) if window else max_kv_len) // tile))
     most = MAX_PREFILL_SPLITS
     if tile == 128:
         most, tiles = MAX_LATENT_SPLITS, 1 << (tiles - 1 + bool(window)).bit_length() if tiles > 1 else 1
+        if rank <= NARROW_LATENT:
+            tiles = max(min(tiles, 16), tiles // 2)
     return int(max(1, min(most, N_SM // (n_items * ctas), tiles)))
 
 

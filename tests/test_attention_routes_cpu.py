@@ -103,3 +103,13 @@ def test_split_counts_of_a_growing_context(n_items, n_kv):
     from hcache_deepspeed_b200.ops.backend import pick_group_splits
     counts = [pick_group_splits(n_items, n_kv, n) for n in range(1, 16385)]
     assert len(set(counts)) <= 3 and counts == sorted(counts) and max(counts) * n_items * n_kv <= 148
+
+
+@pytest.mark.parametrize("rank,keys,window,want", [(512, 4096, 0, 32), (512, 8000, 0, 64), (512, 300, 0, 4), (256, 2000, 0, 16), (256, 4096, 0, 16),
+                                                   (256, 4200, 0, 32), (128, 300, 0, 4), (128, 100, 0, 1), (128, 8000, 0, 32),
+                                                   (128, 16000, 0, 64), (128, 16000, 4096, 32), (128, 9, 4096, 1)])
+def test_splits_of_narrow_latents_get_two_tiles(rank, keys, window, want, monkeypatch):
+    """Wide latents take a split per tile of 128 rows; of narrow ones more than 16 splits are as many as have two tiles."""
+    from hcache_deepspeed_b200.ops import backend, kernels
+    monkeypatch.setattr(kernels, "latent_attention_ctas", lambda *a: (1, 128))
+    assert backend.latent_splits(1, 1, 8, rank, rank + 64, keys, window) == want
